@@ -123,6 +123,7 @@ gms_status multisplit_impl(const uint32_t* kin, const uint32_t* vin, uint32_t* k
   c.bp = to_params(desc);
   c.scratch = static_cast<unsigned char*>(scratch);
   c.stream = stream;
+  c.scratch_bytes = scratch_bytes;
   // Costly identifiers are evaluated once when the scratch has room for a
   // bucket byte per key (the prescan stores them, the postscan reads them).
   if (kind_keeps_bucket_bytes(desc->kind) && scratch_bytes >= g.bytes_full) c.bucket_bytes = c.scratch + g.off_buckets;

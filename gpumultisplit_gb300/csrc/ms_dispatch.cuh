@@ -7,6 +7,7 @@
 #include <atomic>
 
 #include "batch_kernels.cuh"
+#include "fused.cuh"
 #include "histogram_kernels.cuh"
 #include "ms_host.h"
 #include "multisplit_kernels.cuh"
@@ -62,10 +63,96 @@ inline uint32_t persistent_grid(Kernel k, int threads, uint32_t work, std::atomi
 template <int W>
 using ElemT = std::conditional_t<W == 2, uint64_t, uint32_t>;
 
+// When a multisplit runs as one launch (fused.cuh): its tiles are resident all
+// at once, and for pairs with an identifier the three stages evaluate twice
+// (delta, bit field, mask) there are at most FUSED_CHEAP_PAIR_TILES of them.
+// Measured against the three stages replayed from a CUDA graph (us per call):
+//   keys, delta, 256 buckets   10 k 11.4 -> 6.2   260 k 14.9 -> 9.4   1 Mi 15.9 -> 11.9   2.4 M 23.8 -> 19.9
+//   pairs, delta, 32 buckets   10 k  9.1 -> 5.3   260 k 11.2 -> 6.6   1 Mi 13.6 -> 10.3   2.0 M 17.6 -> 17.3
+//   pairs, delta, 64 buckets   1.5 M 17.3 -> 16.0, 2.0 M 19.0 -> 19.6: the line for pairs lies between
+//   pairs, range, 32 buckets   10 k 13.3 -> 7.3   1 Mi 22.4 -> 12.4   2.4 M 26.8 -> 21.6
+// Larger inputs keep the memory busier as three stages, whose tiles are in
+// different phases.
+//
+// Up to FUSED_ADD_MAX counts every block adds up the rows itself (one
+// barrier); above, the columns are scanned first (two barriers).  At 256
+// buckets: 130 k keys (8192 counts) 10.1 against 11.6 us, 260 k keys 11.7
+// against 10.5.
+constexpr uint32_t FUSED_CHEAP_PAIR_TILES = 448;
+constexpr uint32_t FUSED_ADD_MAX = 8192;
+constexpr uint32_t FUSED_CLUSTER_MAX = 16;  // blocks of one cluster (above 8: opt-in)
+
+// Runs a whole multisplit as one launch if the rule above says so and the
+// scratch has room for the counts as [tile][bucket] rows after the matrix and
+// status words (every caller that allocated the reported size has it there:
+// its byte per key).  *launched says whether it did.
+template <class C, class P>
+cudaError_t launch_fused(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, uint32_t n,
+                         const typename P::Params& params, unsigned char* scratch, size_t scratch_bytes,
+                         const Geometry& g, cudaStream_t stream, bool* launched) {
+  static std::atomic<uint64_t> smem_done{0}, cluster_done{0};
+  static std::atomic<int> per_sm{0};
+  *launched = false;
+  if (g.num_tiles > (C::KV && P::CHEAP ? FUSED_CHEAP_PAIR_TILES : FUSED_MAX_TILES)) return cudaSuccess;
+  auto kern = fused_kernel<C, P>;
+  constexpr size_t smem = PostLayout<C, P>::BYTES;
+  cudaError_t e = ensure_smem_limit(kern, smem, smem_done, 2 * C::THREADS * 4);
+  if (e != cudaSuccess) return e;
+  if (persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem) < g.num_tiles) return cudaSuccess;
+  FusedArgs a{};
+  a.num_tiles = g.num_tiles;
+  a.matrix = reinterpret_cast<uint32_t*>(scratch + g.off_matrix);
+  uint32_t blocks = g.num_tiles;
+  if (g.num_tiles > 1) {
+    a.sync = g.num_tiles <= FUSED_CLUSTER_MAX ? FUSED_CLUSTER : FUSED_GRID;
+    const size_t rows_bytes = size_t(g.m) * 4, totals_bytes = size_t(C::B) * 4;
+    if (scratch_bytes < g.off_buckets + rows_bytes + totals_bytes) return cudaSuccess;
+    a.rows = reinterpret_cast<uint32_t*>(scratch + g.off_buckets);
+    if (g.m > FUSED_ADD_MAX) a.totals = reinterpret_cast<uint32_t*>(scratch + g.off_buckets + rows_bytes);
+    if (a.sync == FUSED_CLUSTER)
+      for (blocks = 2; blocks < g.num_tiles; blocks <<= 1) {
+      }
+  }
+  if (blocks > 8 && a.sync == FUSED_CLUSTER) {
+    int dev = 0;
+    e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (!(cluster_done.load(std::memory_order_acquire) & (1ull << (dev & 63)))) {
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return e;
+      cluster_done.fetch_or(1ull << (dev & 63), std::memory_order_acq_rel);
+    }
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(C::THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  if (a.sync == FUSED_CLUSTER) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
+  } else if (a.sync == FUSED_GRID) {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.numAttrs = 1;
+  }
+  cfg.attrs = attr;
+  e = cudaLaunchKernelEx(&cfg, kern, kin, vin, kout, vout, n, a, params, reinterpret_cast<ScratchHeader*>(scratch));
+  if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device has: not all resident
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  *launched = true;
+  return e;
+}
+
 template <class P, int LOGB, bool KV, int KW = 1, int VW = 1>
 cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<KW>* kout, ElemT<VW>* vout,
                               uint32_t n, const typename P::Params& params, unsigned char* scratch, int stages,
-                              cudaStream_t stream, uint8_t* bucket_bytes = nullptr) {
+                              cudaStream_t stream, uint8_t* bucket_bytes = nullptr, size_t scratch_bytes = 0) {
   if constexpr (P::CHEAP) bucket_bytes = nullptr;
   using S = TileShape<LOGB, KV, KW, VW>;
   using C = TileCfg<LOGB, S::WARPS, S::IPT, KV, KW, VW>;
@@ -104,6 +191,14 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
     }
     return cudaSuccess;
   } else {
+  if constexpr (VW == 1) {
+    bool launched = false;
+    if (stages == STAGE_ALL) {
+      const cudaError_t e =
+          launch_fused<C, P>(kin, vin, kout, vout, n, params, scratch, scratch_bytes, g, stream, &launched);
+      if (e != cudaSuccess || launched) return e;
+    }
+  }
   if (stages & STAGE_PRESCAN) {
     static std::atomic<int> per_sm{0};
     auto kern = prescan_kernel<C, P>;
@@ -165,7 +260,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
 template <int KIND, int LOGB, bool KV>
 cudaError_t run_multisplit_t(const MsCall& c, int stages) {
   return launch_multisplit<DescPolicy<KIND, LOGB>, LOGB, KV>(c.kin, c.vin, c.kout, c.vout, c.n, c.bp, c.scratch,
-                                                             stages, c.stream, c.bucket_bytes);
+                                                             stages, c.stream, c.bucket_bytes, c.scratch_bytes);
 }
 
 template <int KIND, bool KV>

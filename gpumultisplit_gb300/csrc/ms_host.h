@@ -131,6 +131,7 @@ struct MsCall {
   unsigned char* scratch = nullptr;  // laid out as make_geometry(n, logb, kv)
   cudaStream_t stream = nullptr;
   uint8_t* bucket_bytes = nullptr;   // in scratch, or null (see launch_multisplit)
+  size_t scratch_bytes = 0;          // bytes at scratch
 };
 
 // Runs the requested stages (a mask of Stage) of one multisplit.  Defined per

@@ -487,6 +487,13 @@ struct GivenOffset {
   __device__ __forceinline__ uint32_t offset(uint32_t, uint32_t) { return goff; }
 };
 
+// Whether a source of offsets is resolved by all threads of the block together
+// (it has a resolve()), after phase 3 and before offset().
+template <class O, class = void>
+struct requires_resolve : std::false_type {};
+template <class O>
+struct requires_resolve<O, std::void_t<decltype(&O::resolve)>> : std::true_type {};
+
 // The default source of a job's offsets: its entries of the scanned count
 // matrix (minus the job's bias in a shared scan).
 struct MatrixOffsets {
@@ -721,6 +728,7 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
   // bucket's output run against n (a corrupt offset can then never cause a
   // store outside the output).
   if constexpr (!Offsets::KNOWN_EARLY) {
+    if constexpr (requires_resolve<Offsets>::value) offs.resolve(tid, my_total);
     if (tid < B) {
       const uint32_t g = offs.offset(tid, my_total);
       if (uint64_t(g) + my_total > n) atomicOr(s_flag, 1u);
