@@ -56,12 +56,28 @@ def _scratch(ctx) -> int | None:
     return _ptr(ctx.d_temp_storage, None)
 
 
-def _stream(stream=None) -> int | None:
-    if stream is not None:
-        return stream if isinstance(stream, int) else stream.cuda_stream
+_current_stream = None  # () -> address of the calling thread's current stream on its current device
+
+
+def _find_current_stream():
+    """The cheapest way torch has: torch.cuda.current_stream() builds a Stream
+    object per call (2.9 us); the raw handle takes 0.3."""
     import torch
 
-    return torch.cuda.current_stream().cuda_stream
+    torch.cuda.current_stream()  # initialises CUDA
+    raw, device = (getattr(torch._C, f, None) for f in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+    if raw is None or device is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(device())
+
+
+def _stream(stream=None) -> int | None:
+    global _current_stream
+    if stream is not None:
+        return stream if isinstance(stream, int) else stream.cuda_stream
+    if _current_stream is None:
+        _current_stream = _find_current_stream()
+    return _current_stream()
 
 
 def _alloc_scratch(nbytes: int):
@@ -93,7 +109,7 @@ class delta_bucket(BucketIdentifier):
     """bucket = key * B >> 32 (B equal-width ranges of the 32-bit key space)."""
 
     def desc(self, num_buckets):
-        return BucketDesc(kind=_lib.GMS_BUCKET_DELTA, num_buckets=num_buckets)
+        return BucketDesc(_lib.GMS_BUCKET_DELTA, num_buckets)
 
     def desc64(self, num_buckets):
         return BucketDesc64(kind=_lib.GMS_BUCKET_DELTA, num_buckets=num_buckets)
@@ -119,7 +135,7 @@ class bits_bucket(BucketIdentifier):
     shift: int = 0
 
     def desc(self, num_buckets):
-        return BucketDesc(kind=_lib.GMS_BUCKET_BITS, num_buckets=num_buckets, shift=int(self.shift))
+        return BucketDesc(_lib.GMS_BUCKET_BITS, num_buckets, int(self.shift))
 
     def desc64(self, num_buckets):
         return BucketDesc64(kind=_lib.GMS_BUCKET_BITS, num_buckets=num_buckets, shift=int(self.shift))
@@ -287,7 +303,8 @@ def _export_offsets(offs, target):
         return None
     import numpy as np
 
-    vals = np.ctypeslib.as_array(offs).tolist()  # far faster than list() on a ctypes array of 64 Ki entries
+    # far faster than list() on a ctypes array of 64 Ki entries, and than np.ctypeslib.as_array on a short one
+    vals = np.frombuffer(offs, np.uint32).tolist()
     if isinstance(target, list):
         target[:] = vals
     return vals

@@ -30,6 +30,7 @@ struct FusedArgs {
   uint32_t* rows;     // the counts as [tile][bucket]
   uint32_t* totals;   // B words for the bucket totals: the columns of rows are scanned, with a
                       // second barrier; null: every block adds up the rows itself
+  uint32_t* starts;   // B words for the bucket starts (pinned host memory), or null
 };
 
 __device__ __forceinline__ void fused_barrier(uint32_t sync) {
@@ -174,7 +175,10 @@ struct FusedOffsets {
       for (uint32_t w = 0; w < SCAN_WARPS; ++w) start += (w < warp) ? s_part[w] : 0u;
     }
     goff = start + before;
-    if (tid < B && tile < a.num_tiles) a.matrix[tid * a.num_tiles + tile] = goff;
+    if (tid < B && tile < a.num_tiles) {
+      a.matrix[tid * a.num_tiles + tile] = goff;
+      if (tile == 0 && a.starts != nullptr) a.starts[tid] = goff;
+    }
   }
   __device__ __forceinline__ uint32_t offset(uint32_t, uint32_t) { return goff; }
 };

@@ -60,6 +60,9 @@ inline uint32_t persistent_grid(Kernel k, int threads, uint32_t work, std::atomi
 // KW / VW: 32-bit words per key / value.  64-bit keys (KW = 2) are identified
 // by the prescan only, which stores every key's bucket in bucket_bytes (then
 // required); their postscan reads those bytes.
+//
+// starts: where the last stage stores the bucket starts (2^LOGB words of
+// pinned host memory), or null.
 template <int W>
 using ElemT = std::conditional_t<W == 2, uint64_t, uint32_t>;
 
@@ -89,7 +92,7 @@ constexpr uint32_t FUSED_CLUSTER_MAX = 16;  // blocks of one cluster (above 8: o
 template <class C, class P>
 cudaError_t launch_fused(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, uint32_t n,
                          const typename P::Params& params, unsigned char* scratch, size_t scratch_bytes,
-                         const Geometry& g, cudaStream_t stream, bool* launched) {
+                         const Geometry& g, cudaStream_t stream, uint32_t* starts, bool* launched) {
   static std::atomic<uint64_t> smem_done{0}, cluster_done{0};
   static std::atomic<int> per_sm{0};
   *launched = false;
@@ -101,6 +104,7 @@ cudaError_t launch_fused(const uint32_t* kin, const uint32_t* vin, uint32_t* kou
   if (persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem) < g.num_tiles) return cudaSuccess;
   FusedArgs a{};
   a.num_tiles = g.num_tiles;
+  a.starts = starts;
   a.matrix = reinterpret_cast<uint32_t*>(scratch + g.off_matrix);
   uint32_t blocks = g.num_tiles;
   if (g.num_tiles > 1) {
@@ -152,7 +156,8 @@ cudaError_t launch_fused(const uint32_t* kin, const uint32_t* vin, uint32_t* kou
 template <class P, int LOGB, bool KV, int KW = 1, int VW = 1>
 cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<KW>* kout, ElemT<VW>* vout,
                               uint32_t n, const typename P::Params& params, unsigned char* scratch, int stages,
-                              cudaStream_t stream, uint8_t* bucket_bytes = nullptr, size_t scratch_bytes = 0) {
+                              cudaStream_t stream, uint8_t* bucket_bytes = nullptr, size_t scratch_bytes = 0,
+                              uint32_t* starts = nullptr) {
   if constexpr (P::CHEAP) bucket_bytes = nullptr;
   using S = TileShape<LOGB, KV, KW, VW>;
   using C = TileCfg<LOGB, S::WARPS, S::IPT, KV, KW, VW>;
@@ -187,7 +192,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
       const uint32_t wave = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem);
       const uint32_t dist = (GMS_PREFETCH_WAVES * wave) / 4u;
       return launch_after_previous(kern, dim3(g.num_tiles), dim3(C::THREADS), smem, stream, kin, vin, kout, vout, n,
-                                   g.num_tiles, matrix, params, hdr, dist, bucket_bytes);
+                                   g.num_tiles, matrix, params, hdr, dist, bucket_bytes, starts);
     }
     return cudaSuccess;
   } else {
@@ -195,7 +200,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
     bool launched = false;
     if (stages == STAGE_ALL) {
       const cudaError_t e =
-          launch_fused<C, P>(kin, vin, kout, vout, n, params, scratch, scratch_bytes, g, stream, &launched);
+          launch_fused<C, P>(kin, vin, kout, vout, n, params, scratch, scratch_bytes, g, stream, starts, &launched);
       if (e != cudaSuccess || launched) return e;
     }
   }
@@ -224,7 +229,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
       const uint32_t wave = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem);
       const uint32_t dist = (GMS_PREFETCH_WAVES * wave) / 4u;
       return launch_after_previous(kern, dim3(g.num_tiles), dim3(C::THREADS), smem, stream, kin, vin, kout, vout, n,
-                                   g.num_tiles, matrix, params, hdr, dist, bucket_bytes);
+                                   g.num_tiles, matrix, params, hdr, dist, bucket_bytes, starts);
     }
   }
   if ((stages & STAGE_POSTSCAN) && P::USES_SMEM) {
@@ -237,7 +242,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
     if (e != cudaSuccess) return e;
     const uint32_t grid = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem);
     return launch_after_previous(kern, dim3(grid), dim3(C::THREADS), smem, stream, kin, vin, kout, vout, n,
-                                 g.num_tiles, matrix, params, hdr);
+                                 g.num_tiles, matrix, params, hdr, starts);
   }
   if (stages & STAGE_POSTSCAN) {
     static std::atomic<uint64_t> smem_done{0};
@@ -250,7 +255,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
     const uint32_t wave = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem);
     const uint32_t dist = (GMS_PREFETCH_WAVES * wave) / 4u;
     e = launch_after_previous(kern, dim3(g.num_tiles), dim3(C::THREADS), smem, stream, kin, vin, kout, vout, n,
-                              g.num_tiles, matrix, params, hdr, dist, static_cast<const uint8_t*>(nullptr));
+                              g.num_tiles, matrix, params, hdr, dist, static_cast<const uint8_t*>(nullptr), starts);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -260,7 +265,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
 template <int KIND, int LOGB, bool KV>
 cudaError_t run_multisplit_t(const MsCall& c, int stages) {
   return launch_multisplit<DescPolicy<KIND, LOGB>, LOGB, KV>(c.kin, c.vin, c.kout, c.vout, c.n, c.bp, c.scratch,
-                                                             stages, c.stream, c.bucket_bytes, c.scratch_bytes);
+                                                             stages, c.stream, c.bucket_bytes, c.scratch_bytes, c.starts);
 }
 
 template <int KIND, bool KV>
@@ -295,10 +300,10 @@ cudaError_t run_multisplit_wide_t(const MsCallWide& c, int stages) {
   if constexpr (KW == 2)
     return launch_multisplit<DescPolicy64<KIND, LOGB>, LOGB, KV, KW, VW>(kin, vin, kout, vout, c.n, c.bp64,
                                                                            c.scratch, stages, c.stream,
-                                                                           c.bucket_bytes);
+                                                                           c.bucket_bytes, 0, c.starts);
   else
     return launch_multisplit<DescPolicy<KIND, LOGB>, LOGB, KV, KW, VW>(kin, vin, kout, vout, c.n, c.bp, c.scratch,
-                                                                         stages, c.stream, c.bucket_bytes);
+                                                                         stages, c.stream, c.bucket_bytes, 0, c.starts);
 }
 
 template <int KIND, int LOGB>
@@ -492,7 +497,8 @@ cudaError_t digit_postscan_t(const DigitPass& c) {
   const uint32_t wave = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem);
   const uint32_t dist = (GMS_PREFETCH_WAVES * wave) / 4u;
   return launch_after_previous(kern, dim3(g.num_tiles), dim3(C::THREADS), smem, c.stream, c.kin, c.vin, c.kout,
-                               c.vout, c.n, g.num_tiles, matrix, c.bp, hdr, dist, c.bucket_bytes);
+                               c.vout, c.n, g.num_tiles, matrix, c.bp, hdr, dist, c.bucket_bytes,
+                               static_cast<uint32_t*>(nullptr));
 }
 
 #define GMS_DIGIT_SWITCH(FN, ...)                                 \

@@ -132,6 +132,7 @@ struct MsCall {
   cudaStream_t stream = nullptr;
   uint8_t* bucket_bytes = nullptr;   // in scratch, or null (see launch_multisplit)
   size_t scratch_bytes = 0;          // bytes at scratch
+  uint32_t* starts = nullptr;        // pinned host memory for 2^logb bucket starts, or null
 };
 
 // Runs the requested stages (a mask of Stage) of one multisplit.  Defined per
@@ -157,6 +158,7 @@ struct MsCallWide {
   unsigned char* scratch = nullptr;  // laid out as make_geometry(n, logb, kv, kw, vw)
   cudaStream_t stream = nullptr;
   uint8_t* bucket_bytes = nullptr;
+  uint32_t* starts = nullptr;        // pinned host memory for 2^logb bucket starts, or null
 };
 
 // Defined per identifier kind in inst_wide.cu (compiled once per kind).

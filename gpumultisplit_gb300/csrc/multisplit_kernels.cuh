@@ -944,15 +944,24 @@ __device__ __forceinline__ void postscan_run(uint32_t first, uint32_t last, uint
   }
 }
 
+// The bucket starts (column 0 of the scanned matrix), stored by the block of
+// tile 0 where the caller wants them: pinned host memory (capi.cu).
+__device__ __forceinline__ void store_starts(uint32_t* starts, const uint32_t* offsets, uint32_t num_tiles,
+                                             uint32_t num_buckets) {
+  if (starts != nullptr && threadIdx.x < num_buckets) starts[threadIdx.x] = offsets[threadIdx.x * num_tiles];
+}
+
 // Plain postscan: one block per tile of one multisplit.  GIVEN: the buckets
 // come from bucket_bytes (written by the prescan).
 template <class C, class P, bool GIVEN = false>
 __global__ void __launch_bounds__(C::THREADS, (PostLayout<C, P, GIVEN>::MIN_BLOCKS)) postscan_kernel(
     const typename C::KT* __restrict__ kin, const typename C::VT* __restrict__ vin, typename C::KT* __restrict__ kout,
     typename C::VT* __restrict__ vout, uint32_t n, uint32_t num_tiles, const uint32_t* __restrict__ offsets,
-    typename P::Params bp, ScratchHeader* hdr, uint32_t prefetch_dist, const uint8_t* __restrict__ bucket_bytes) {
+    typename P::Params bp, ScratchHeader* hdr, uint32_t prefetch_dist, const uint8_t* __restrict__ bucket_bytes,
+    uint32_t* starts) {
   extern __shared__ __align__(128) unsigned char smem[];
   griddep_wait();  // launched while the scan finishes: its offsets are complete past this point
+  if (blockIdx.x == 0) store_starts(starts, offsets, num_tiles, C::B);
   const TileJob<typename P::Params, typename C::KT, typename C::VT> job{kin,        vin,     kout, vout,
                                         n,          num_tiles, blockIdx.x, offsets,
                                         0u,         prefetch_dist != 0 ? blockIdx.x + prefetch_dist : ~0u,
@@ -968,9 +977,10 @@ template <class C, class P>
 __global__ void __launch_bounds__(C::THREADS, (PostLayout<C, P>::MIN_BLOCKS)) postscan_persistent_kernel(
     const typename C::KT* __restrict__ kin, const typename C::VT* __restrict__ vin, typename C::KT* __restrict__ kout,
     typename C::VT* __restrict__ vout, uint32_t n, uint32_t num_tiles, const uint32_t* __restrict__ offsets,
-    typename P::Params bp, ScratchHeader* hdr) {
+    typename P::Params bp, ScratchHeader* hdr, uint32_t* starts) {
   extern __shared__ __align__(128) unsigned char smem[];
   griddep_wait();  // launched while the scan finishes: its offsets are complete past this point
+  if (blockIdx.x == 0) store_starts(starts, offsets, num_tiles, C::B);
   postscan_run<C, P>(
       blockIdx.x, num_tiles, gridDim.x,
       [&](uint32_t t, uint32_t prefetch) {
