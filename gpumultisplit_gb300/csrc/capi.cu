@@ -218,14 +218,15 @@ struct SortLayout {
   size_t ms_bytes;   // multisplit scratch (largest over the schedule's digit widths)
   size_t off_keys;   // ping-pong keys
   size_t off_vals;   // ping-pong values
-  size_t bytes;
+  size_t bytes;      // what a sort needs
+  size_t bytes_full;  // plus the count rows of a one-launch sort (what the scratch size calls report)
 };
 
 SortLayout sort_layout(uint32_t n, bool kv, const SortSchedule& sch) {
   SortLayout L;
   L.ms_bytes = 0;
   if (sch.passes == 0) {  // nothing to sort: the input is copied
-    L.off_keys = L.off_vals = L.bytes = 0;
+    L.off_keys = L.off_vals = L.bytes = L.bytes_full = 0;
     return L;
   }
   for (int p = 0; p < sch.passes; ++p) {
@@ -244,7 +245,52 @@ SortLayout sort_layout(uint32_t n, bool kv, const SortSchedule& sch) {
   L.off_keys = align_up(L.ms_bytes, 256);
   L.off_vals = align_up(L.off_keys + size_t(n) * 4, 256);
   L.bytes = kv ? align_up(L.off_vals + size_t(n) * 4, 256) : L.off_vals;
+  L.bytes_full = L.bytes + align_up(fused_sort_rows_bytes(n), 256);
   return L;
+}
+
+// Whether a sort's buffers allow any schedule: no input array shares a byte
+// with an output array (an even number of passes may otherwise run in place)
+// and the outputs are apart.
+bool sort_buffers_apart(const void* kin, const void* kout, const void* vin, const void* vout, uint32_t n, size_t kb,
+                        size_t vb) {
+  return !overlaps(kin, kout, n, kb, kb) && !overlaps(kin, vout, n, kb, vb) && !overlaps(vin, kout, n, vb, kb) &&
+         !overlaps(vin, vout, n, vb, vb) && !overlaps(kout, vout, n, kb, vb);
+}
+
+// Runs a sort as one launch when it can (inst_sort.cu); the stable order by the
+// key bits is the same whatever the digits.  The count rows go behind the
+// ping-pong buffers when the caller's scratch reaches that far, else (and for
+// 64-bit keys, whose bucket bytes leave the room) into the passes' own scratch.
+gms_status sort_one_launch(const void* kin, void* kout, const void* vin, void* vout, uint32_t n, int key_bytes,
+                           int value_bytes, const SortSchedule& sch, const SortLayout& L, unsigned char* scratch,
+                           size_t scratch_bytes, void* tk, void* tv, cudaStream_t stream, bool* launched) {
+  *launched = false;
+  if ((reinterpret_cast<uintptr_t>(scratch) & 255u) != 0) return GMS_SUCCESS;
+  auto aligned = [](const void* p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & uintptr_t(bytes - 1)) == 0; };
+  if (!aligned(kin, key_bytes) || !aligned(kout, key_bytes)) return GMS_SUCCESS;
+  if (value_bytes != 0 && (!aligned(vin, value_bytes) || !aligned(vout, value_bytes))) return GMS_SUCCESS;
+  if (!sort_buffers_apart(kin, kout, vin, vout, n, size_t(key_bytes), size_t(value_bytes))) return GMS_SUCCESS;
+  FusedSortCall c;
+  c.kin = kin;
+  c.vin = vin;
+  c.kout = kout;
+  c.vout = vout;
+  c.tk = tk;
+  c.tv = tv;
+  c.n = n;
+  c.key_bytes = key_bytes;
+  c.value_bytes = value_bytes;
+  c.begin_bit = sch.shift[0];
+  c.end_bit = sch.shift[sch.passes - 1];
+  for (uint32_t b = sch.buckets[sch.passes - 1]; b > 1; b >>= 1) ++c.end_bit;
+  c.hdr = reinterpret_cast<ScratchHeader*>(scratch);
+  const size_t rows = fused_sort_rows_bytes(n);
+  const bool behind = key_bytes == 4 && scratch_bytes >= L.bytes + rows;
+  c.rows = scratch + (behind ? L.bytes : sizeof(ScratchHeader));
+  c.rows_bytes = behind ? rows : L.ms_bytes - sizeof(ScratchHeader);
+  c.stream = stream;
+  return cuda_status(run_fused_sort(c, launched));
 }
 
 // Which way the 32-bit sorts run their digits (gms_sort_set_method).
@@ -294,6 +340,12 @@ gms_status sort_run(const uint32_t* kin, uint32_t* kout, const uint32_t* vin, ui
     for (int p = 0; p < sch.passes; ++p) valid_buckets(sch.buckets[p], reinterpret_cast<int*>(&logb[p]));
     return cuda_status(run_onesweep_sort(kin, kout, kv ? vin : nullptr, kv ? vout : nullptr, n, kv, sch.passes,
                                          sch.shift, logb, base, tk, tv, stream));
+  }
+  if (g_sort_method.load(std::memory_order_relaxed) == GMS_SORT_AUTO) {
+    bool launched = false;
+    const gms_status st = sort_one_launch(kin, kout, kv ? vin : nullptr, kv ? vout : nullptr, n, 4, kv ? 4 : 0, sch,
+                                          L, base, scratch_bytes, tk, tv, stream, &launched);
+    if (st != GMS_SUCCESS || launched) return st;
   }
   const uint32_t* ki = kin;
   const uint32_t* vi = vin;
@@ -590,6 +642,7 @@ gms_status multisplit_wide_impl(const void* kin, const void* vin, void* kout, vo
   c.vw = vw;
   c.scratch = static_cast<unsigned char*>(scratch);
   c.stream = stream;
+  c.scratch_bytes = scratch_bytes;
   c.starts = starts;
   if (key_bytes == 8) {
     c.bp64 = to_params64(desc);
@@ -607,7 +660,7 @@ SortLayout sort_layout_wide(uint32_t n, int key_bytes, int value_bytes, const So
   SortLayout L;
   L.ms_bytes = 0;
   if (sch.passes == 0) {
-    L.off_keys = L.off_vals = L.bytes = 0;
+    L.off_keys = L.off_vals = L.bytes = L.bytes_full = 0;
     return L;
   }
   const bool kv = value_bytes != 0;
@@ -621,6 +674,8 @@ SortLayout sort_layout_wide(uint32_t n, int key_bytes, int value_bytes, const So
   L.off_keys = align_up(L.ms_bytes, 256);
   L.off_vals = align_up(L.off_keys + size_t(n) * key_bytes, 256);
   L.bytes = kv ? align_up(L.off_vals + size_t(n) * value_bytes, 256) : L.off_vals;
+  // 64-bit keys have the room in front, in their bucket bytes
+  L.bytes_full = L.bytes + (key_bytes == 4 ? align_up(fused_sort_rows_bytes(n), 256) : 0);
   return L;
 }
 
@@ -646,6 +701,10 @@ gms_status sort_wide_run(const void* kin, void* kout, const void* vin, void* vou
   auto* base = static_cast<unsigned char*>(scratch);
   void* tk = base + L.off_keys;
   void* tv = kv ? base + L.off_vals : nullptr;
+  bool launched = false;
+  const gms_status one = sort_one_launch(kin, kout, kv ? vin : nullptr, kv ? vout : nullptr, n, key_bytes, value_bytes,
+                                         sch, L, base, scratch_bytes, tk, tv, stream, &launched);
+  if (one != GMS_SUCCESS || launched) return one;
   const void* ki = kin;
   const void* vi = vin;
   for (int p = 0; p < sch.passes; ++p) {
@@ -826,7 +885,7 @@ gms_status gms_sort_get_method(int* method) {
 gms_status gms_sort_scratch_bytes(uint32_t max_elements, int digit_bits, int key_value, size_t* bytes) {
   SortSchedule sch;
   if (bytes == nullptr || !sort_schedule(digit_bits, &sch)) return GMS_ERROR_INVALID_VALUE;
-  *bytes = sort_layout(max_elements, key_value != 0, sch).bytes;
+  *bytes = sort_layout(max_elements, key_value != 0, sch).bytes_full;
   return GMS_SUCCESS;
 }
 
@@ -846,7 +905,7 @@ gms_status gms_sort_bits_scratch_bytes(uint32_t max_elements, int begin_bit, int
                                       int key_value, size_t* bytes) {
   SortSchedule sch;
   if (bytes == nullptr || !bit_schedule(begin_bit, end_bit, digit_bits, &sch)) return GMS_ERROR_INVALID_VALUE;
-  *bytes = sort_layout(max_elements, key_value != 0, sch).bytes;
+  *bytes = sort_layout(max_elements, key_value != 0, sch).bytes_full;
   return GMS_SUCCESS;
 }
 
@@ -1000,7 +1059,7 @@ gms_status gms_sort_wide_scratch_bytes(uint32_t max_elements, int key_bytes, int
   if (bytes == nullptr || !valid_widths(key_bytes, value_bytes) ||
       !bit_schedule(begin_bit, end_bit, digit_bits, &sch, 8 * key_bytes))
     return GMS_ERROR_INVALID_VALUE;
-  *bytes = sort_layout_wide(max_elements, key_bytes, value_bytes, sch).bytes;
+  *bytes = sort_layout_wide(max_elements, key_bytes, value_bytes, sch).bytes_full;
   return GMS_SUCCESS;
 }
 

@@ -26,12 +26,18 @@ enum FusedSync : uint32_t {
 struct FusedArgs {
   uint32_t num_tiles;
   uint32_t sync;      // FusedSync
-  uint32_t* matrix;   // the count matrix, [bucket][tile]; holds global offsets afterwards
-  uint32_t* rows;     // the counts as [tile][bucket]
+  uint32_t* matrix;   // the count matrix, [bucket][tile]; holds global offsets afterwards (null: not kept)
+  uint32_t* rows;     // the counts as [tile][bucket]; null: the blocks of a cluster read each other's
+                      // shared memory
   uint32_t* totals;   // B words for the bucket totals: the columns of rows are scanned, with a
                       // second barrier; null: every block adds up the rows itself
   uint32_t* starts;   // B words for the bucket starts (pinned host memory), or null
 };
+
+// Second half of the cluster barrier that FusedOffsets::resolve() arrives at.
+__device__ __forceinline__ void fused_counts_read(const FusedArgs& a) {
+  if (a.sync == FUSED_CLUSTER && a.rows == nullptr) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
 
 __device__ __forceinline__ void fused_barrier(uint32_t sync) {
   if (sync == FUSED_GRID) {
@@ -41,6 +47,15 @@ __device__ __forceinline__ void fused_barrier(uint32_t sync) {
   } else {
     __syncthreads();
   }
+}
+
+// A word of another block's shared memory in the same cluster: `local` is the
+// word's address in this block's.
+__device__ __forceinline__ uint32_t ld_cluster_u32(const uint32_t* local, uint32_t rank) {
+  uint32_t addr, v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(local)), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
 }
 
 // The most tiles one launch can hold: the column scan keeps a thread's rows in
@@ -59,11 +74,14 @@ struct FusedOffsets {
   FusedArgs a;
   uint32_t tile;
   uint32_t* s_part;  // 2 * THREADS words
+  uint32_t* s_cnt;   // B words: this block's counts, which the blocks of its cluster read
   uint32_t goff;
 
   __device__ __forceinline__ void aggregate(uint32_t b, uint32_t total) {
-    if (a.sync == FUSED_ONE_TILE || tile >= a.num_tiles) return;
-    a.rows[tile * B + b] = total;
+    if (a.rows == nullptr)
+      s_cnt[b] = total;
+    else if (tile < a.num_tiles)
+      a.rows[tile * B + b] = total;
   }
 
   __device__ __forceinline__ void resolve(uint32_t tid, uint32_t my_total) {
@@ -80,10 +98,13 @@ struct FusedOffsets {
       total = 0;
 #pragma unroll 8
       for (uint32_t t = tid / B; t < a.num_tiles; t += R) {
-        const uint32_t v = __ldcg(a.rows + t * B + b);
+        const uint32_t v = a.rows == nullptr ? ld_cluster_u32(s_cnt + b, t) : __ldcg(a.rows + t * B + b);
         total += v;
         before += t < tile ? v : 0u;
       }
+      // No block leaves (or counts again) before the others have read its counts:
+      // fused_counts_read() waits for this arrival.
+      if (a.rows == nullptr) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
       if constexpr (B < 32) {
 #pragma unroll
         for (uint32_t d = B; d < 32; d <<= 1) {
@@ -175,7 +196,7 @@ struct FusedOffsets {
       for (uint32_t w = 0; w < SCAN_WARPS; ++w) start += (w < warp) ? s_part[w] : 0u;
     }
     goff = start + before;
-    if (tid < B && tile < a.num_tiles) {
+    if (tid < B && tile < a.num_tiles && a.matrix != nullptr) {
       a.matrix[tid * a.num_tiles + tile] = goff;
       if (tile == 0 && a.starts != nullptr) a.starts[tid] = goff;
     }
@@ -183,36 +204,37 @@ struct FusedOffsets {
   __device__ __forceinline__ uint32_t offset(uint32_t, uint32_t) { return goff; }
 };
 
-// Blocks per SM the fused kernel is register-budgeted for (64 registers).
-constexpr int FUSED_BLOCKS = 4;
-
-// Stage cnt elements at src into shared memory, all loads in flight together:
-// 16-byte loads and up to three single elements when src is 16-byte aligned,
-// single elements otherwise.
-template <int THREADS, int IPT>
-__device__ __forceinline__ void stage_tile(uint32_t* dst, const uint32_t* __restrict__ src, uint32_t cnt) {
+// Stage cnt 32- or 64-bit elements at src into shared memory, all loads in
+// flight together: 16-byte loads and the last few elements singly when src is
+// 16-byte aligned, single elements otherwise.  Through L2: a sort's later
+// passes read what other blocks of the launch wrote.
+template <int THREADS, int IPT, class T>
+__device__ __forceinline__ void stage_tile(T* dst, const T* src, uint32_t cnt) {
+  constexpr uint32_t EV = 16 / sizeof(T);  // elements per vector
+  constexpr int NV = IPT / int(EV);
+  static_assert(IPT % int(EV) == 0, "whole vectors per thread");
   const uint32_t tid = threadIdx.x;
   if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
-    const uint32_t nv = cnt / 4u;
-    uint4 v[IPT / 4];
+    const uint32_t nv = cnt / EV;
+    uint4 v[NV];
 #pragma unroll
-    for (int k = 0; k < IPT / 4; ++k) {
+    for (int k = 0; k < NV; ++k) {
       const uint32_t i = uint32_t(k) * THREADS + tid;
-      v[k] = i < nv ? ld_nc_v4(src + i * 4u) : make_uint4(0u, 0u, 0u, 0u);
+      v[k] = i < nv ? __ldcg(reinterpret_cast<const uint4*>(src + i * EV)) : make_uint4(0u, 0u, 0u, 0u);
     }
-    const uint32_t tail = 4u * nv + tid;
-    if (tail < cnt) dst[tail] = src[tail];
+    const uint32_t tail = EV * nv + tid;
+    if (tail < cnt) dst[tail] = __ldcg(src + tail);
 #pragma unroll
-    for (int k = 0; k < IPT / 4; ++k) {
+    for (int k = 0; k < NV; ++k) {
       const uint32_t i = uint32_t(k) * THREADS + tid;
-      if (i < nv) *reinterpret_cast<uint4*>(dst + i * 4u) = v[k];
+      if (i < nv) *reinterpret_cast<uint4*>(dst + i * EV) = v[k];
     }
   } else {
-    uint32_t v[IPT];
+    T v[IPT];
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
       const uint32_t i = uint32_t(k) * THREADS + tid;
-      v[k] = i < cnt ? src[i] : 0u;
+      v[k] = i < cnt ? __ldcg(src + i) : T(0);
     }
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
@@ -222,39 +244,137 @@ __device__ __forceinline__ void stage_tile(uint32_t* dst, const uint32_t* __rest
   }
 }
 
+// Blocks per SM the fused kernel is register-budgeted for: four (64
+// registers), fewer where 64-bit elements fill the shared memory first.
 template <class C, class P>
-__global__ void __launch_bounds__(C::THREADS, FUSED_BLOCKS) fused_kernel(
-    const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
-    uint32_t* __restrict__ vout, uint32_t n, FusedArgs a, typename P::Params bp, ScratchHeader* hdr) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  using L = PostLayout<C, P>;
-  static_assert(C::KW == 1 && C::VW == 1, "32-bit elements");
-  __shared__ uint32_t s_part[2 * C::THREADS];
+constexpr int fused_blocks() {
+  return C::WIDE && PostLayout<C, P, C::KW == 2>::MIN_BLOCKS < 4 ? PostLayout<C, P, C::KW == 2>::MIN_BLOCKS : 4;
+}
+
+// One block's tile of one multisplit among the blocks of its launch.
+// 64-bit keys: the tile's buckets are computed once, as bytes, from the staged
+// keys (the GIVEN form of the tile's work), with the identifier's state at
+// s_ident.
+template <class C, class P>
+__device__ __forceinline__ void fused_tile(const typename C::KT* kin, const typename C::VT* vin, typename C::KT* kout,
+                                           typename C::VT* vout, uint32_t n, const FusedArgs& a,
+                                           const typename P::Params& bp, ScratchHeader* hdr, unsigned char* smem,
+                                           uint32_t* s_part, uint32_t* s_cnt, uint32_t* s_ident) {
+  constexpr bool GIVEN = C::KW == 2;
+  using L = PostLayout<C, P, GIVEN>;
+  using KT = typename C::KT;
+  using VT = typename C::VT;
   const uint32_t tid = threadIdx.x;
   const uint32_t tile = blockIdx.x;  // a cluster may have blocks past the last tile: empty tiles
   const uint32_t base = tile < a.num_tiles ? tile * C::TILE : n;
   const uint32_t cnt = min(C::TILE, n - base);
-  if (tile == 0 && tid == 0) {
-    hdr->error = 0u;
-    hdr->error_info = 0u;
-    hdr->ticket = 0u;
-    hdr->wait_limit_us = 0u;
-  }
   if (tid == 0) *reinterpret_cast<uint32_t*>(smem + L::OFF_FLAG) = 0u;
-  stage_tile<C::THREADS, C::IPT>(reinterpret_cast<uint32_t*>(smem + L::OFF_K), kin + base, cnt);
-  if constexpr (C::KV) stage_tile<C::THREADS, C::IPT>(reinterpret_cast<uint32_t*>(smem + L::OFF_V), vin + base, cnt);
-  P::prepare(reinterpret_cast<uint32_t*>(smem + L::OFF_SPLIT), bp);
+  KT* s_k = reinterpret_cast<KT*>(smem + L::OFF_K);
+  stage_tile<C::THREADS, C::IPT>(s_k, kin + base, cnt);
+  if constexpr (C::KV) stage_tile<C::THREADS, C::IPT>(reinterpret_cast<VT*>(smem + L::OFF_V), vin + base, cnt);
+  uint32_t* s_state = GIVEN ? s_ident : reinterpret_cast<uint32_t*>(smem + L::OFF_SPLIT);
+  P::prepare(s_state, bp);
   if constexpr (C::LOGB > 5) {
     constexpr uint32_t WORDS = L::SUBWARPS * C::WB * C::WS * sizeof(typename L::WhT) / 4;
     uint32_t* s_wh = reinterpret_cast<uint32_t*>(smem + L::OFF_WH);
     for (uint32_t i = tid; i < WORDS; i += C::THREADS) s_wh[i] = 0u;
   }
   __syncthreads();
-  FusedOffsets<C> offs{a, tile, s_part, 0u};
+  if constexpr (GIVEN) {
+    const typename P::Id ident = P::make(bp, s_state);
+    uint8_t* s_rb = reinterpret_cast<uint8_t*>(smem + L::OFF_RB);
+    for (uint32_t i = tid; i < cnt; i += C::THREADS) s_rb[i] = uint8_t(ident(s_k[i]));
+    __syncthreads();
+  }
+  FusedOffsets<C> offs{a, tile, s_part, s_cnt, 0u};
   if (cnt == C::TILE)
-    postscan_tile<C, P, true, false, FusedOffsets<C>>(kout, vout, n, cnt, offs, bp, hdr, smem);
+    postscan_tile<C, P, true, GIVEN, FusedOffsets<C>>(kout, vout, n, cnt, offs, bp, hdr, smem);
   else
-    postscan_tile<C, P, false, false, FusedOffsets<C>>(kout, vout, n, cnt, offs, bp, hdr, smem);
+    postscan_tile<C, P, false, GIVEN, FusedOffsets<C>>(kout, vout, n, cnt, offs, bp, hdr, smem);
+  fused_counts_read(a);
+}
+
+__device__ __forceinline__ void fused_reset_header(ScratchHeader* hdr) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    hdr->error = 0u;
+    hdr->error_info = 0u;
+    hdr->ticket = 0u;
+    hdr->wait_limit_us = 0u;
+  }
+}
+
+// Shared words of a 64-bit identifier's state (32-bit ones keep theirs in the
+// tile's layout).
+template <class C, class P>
+constexpr uint32_t fused_ident_words() {
+  return C::KW == 2 ? P::SMEM_WORDS : 1u;
+}
+
+template <class C, class P>
+__global__ void __launch_bounds__(C::THREADS, (fused_blocks<C, P>())) fused_kernel(
+    const typename C::KT* __restrict__ kin, const typename C::VT* __restrict__ vin, typename C::KT* __restrict__ kout,
+    typename C::VT* __restrict__ vout, uint32_t n, FusedArgs a, typename P::Params bp, ScratchHeader* hdr) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint32_t s_part[2 * C::THREADS];
+  __shared__ uint32_t s_cnt[C::B];
+  __shared__ __align__(16) uint32_t s_ident[fused_ident_words<C, P>()];
+  fused_reset_header(hdr);
+  fused_tile<C, P>(kin, vin, kout, vout, n, a, bp, hdr, smem, s_part, s_cnt, s_ident);
+}
+
+// A digit of the key, for the sort below: at most 2^LOGB values.
+struct FieldParams {
+  uint32_t shift;
+  uint32_t mask;
+};
+struct FieldId {
+  FieldParams p;
+  template <class K>
+  __device__ __forceinline__ uint32_t operator()(K key) const {
+    return uint32_t(key >> p.shift) & p.mask;
+  }
+};
+template <bool CHEAP_>
+struct FieldPolicy {
+  using Params = FieldParams;
+  using Id = FieldId;
+  static constexpr bool CHEAP = CHEAP_;
+  static constexpr bool USES_SMEM = false;
+  static constexpr uint32_t SMEM_WORDS = 1;
+  __device__ __forceinline__ static void prepare(uint32_t*, const Params&) {}
+  __device__ __forceinline__ static Id make(const Params& p, const uint32_t*) { return Id{p}; }
+};
+
+// A whole LSD sort in one launch: one multisplit per digit of at most `digit`
+// bits over key bits [begin, end), ping-ponging so that the last lands in
+// kout/vout, with a barrier between passes.
+struct FusedDigits {
+  uint32_t begin, end, digit;
+};
+
+template <class C, class P>
+__global__ void __launch_bounds__(C::THREADS, (fused_blocks<C, P>())) fused_sort_kernel(
+    const typename C::KT* kin, const typename C::VT* vin, typename C::KT* kout, typename C::VT* vout,
+    typename C::KT* tk, typename C::VT* tv, uint32_t n, FusedArgs a, FusedDigits d, ScratchHeader* hdr) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint32_t s_part[2 * C::THREADS];
+  __shared__ uint32_t s_cnt[C::B];
+  __shared__ uint32_t s_ident[1];
+  fused_reset_header(hdr);
+  const uint32_t passes = (d.end - d.begin + d.digit - 1) / d.digit;
+  const typename C::KT* ki = kin;
+  const typename C::VT* vi = vin;
+  for (uint32_t p = 0; p < passes; ++p) {
+    const bool to_out = ((passes - 1 - p) & 1u) == 0u;
+    typename C::KT* ko = to_out ? kout : tk;
+    typename C::VT* vo = to_out ? vout : tv;
+    const uint32_t shift = d.begin + p * d.digit;
+    const FieldParams bp{shift, (1u << min(d.digit, d.end - shift)) - 1u};
+    if (p != 0) fused_barrier(a.sync);  // the previous pass's output is complete, its counts are read
+    fused_tile<C, P>(ki, vi, ko, vo, n, a, bp, hdr, smem, s_part, s_cnt, s_ident);
+    ki = ko;
+    vi = vo;
+  }
 }
 
 }  // namespace gms

@@ -85,72 +85,133 @@ constexpr uint32_t FUSED_CHEAP_PAIR_TILES = 448;
 constexpr uint32_t FUSED_ADD_MAX = 8192;
 constexpr uint32_t FUSED_CLUSTER_MAX = 16;  // blocks of one cluster (above 8: opt-in)
 
-// Runs a whole multisplit as one launch if the rule above says so and the
-// scratch has room for the counts as [tile][bucket] rows after the matrix and
-// status words (every caller that allocated the reported size has it there:
-// its byte per key).  *launched says whether it did.
-template <class C, class P>
-cudaError_t launch_fused(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, uint32_t n,
-                         const typename P::Params& params, unsigned char* scratch, size_t scratch_bytes,
-                         const Geometry& g, cudaStream_t stream, uint32_t* starts, bool* launched) {
-  static std::atomic<uint64_t> smem_done{0}, cluster_done{0};
-  static std::atomic<int> per_sm{0};
-  *launched = false;
-  if (g.num_tiles > (C::KV && P::CHEAP ? FUSED_CHEAP_PAIR_TILES : FUSED_MAX_TILES)) return cudaSuccess;
-  auto kern = fused_kernel<C, P>;
-  constexpr size_t smem = PostLayout<C, P>::BYTES;
-  cudaError_t e = ensure_smem_limit(kern, smem, smem_done, 2 * C::THREADS * 4);
+// What a one-launch kernel remembers per process (per device where it matters).
+struct FusedKernelState {
+  std::atomic<uint64_t> smem_done{0}, cluster_done{0};
+  std::atomic<int> per_sm{0};
+};
+
+// Prepares `kern` to run num_tiles tiles in one launch: its limits, the form of
+// its barrier (a->sync) and the launch configuration.  *fits: all tiles are
+// resident at once.
+template <class C, class Kernel>
+cudaError_t fused_config(Kernel kern, size_t smem, size_t static_smem, uint32_t num_tiles, FusedKernelState& state,
+                         cudaStream_t stream, FusedArgs* a, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr,
+                         bool* fits) {
+  *fits = false;
+  cudaError_t e = ensure_smem_limit(kern, smem, state.smem_done, static_smem);
   if (e != cudaSuccess) return e;
-  if (persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem) < g.num_tiles) return cudaSuccess;
-  FusedArgs a{};
-  a.num_tiles = g.num_tiles;
-  a.starts = starts;
-  a.matrix = reinterpret_cast<uint32_t*>(scratch + g.off_matrix);
-  uint32_t blocks = g.num_tiles;
-  if (g.num_tiles > 1) {
-    a.sync = g.num_tiles <= FUSED_CLUSTER_MAX ? FUSED_CLUSTER : FUSED_GRID;
-    const size_t rows_bytes = size_t(g.m) * 4, totals_bytes = size_t(C::B) * 4;
-    if (scratch_bytes < g.off_buckets + rows_bytes + totals_bytes) return cudaSuccess;
-    a.rows = reinterpret_cast<uint32_t*>(scratch + g.off_buckets);
-    if (g.m > FUSED_ADD_MAX) a.totals = reinterpret_cast<uint32_t*>(scratch + g.off_buckets + rows_bytes);
-    if (a.sync == FUSED_CLUSTER)
-      for (blocks = 2; blocks < g.num_tiles; blocks <<= 1) {
-      }
-  }
-  if (blocks > 8 && a.sync == FUSED_CLUSTER) {
+  if (persistent_grid(kern, C::THREADS, num_tiles, state.per_sm, smem) < num_tiles) return cudaSuccess;
+  a->num_tiles = num_tiles;
+  a->sync = num_tiles == 1 ? FUSED_ONE_TILE : num_tiles <= FUSED_CLUSTER_MAX ? FUSED_CLUSTER : FUSED_GRID;
+  uint32_t blocks = num_tiles;
+  cfg->attrs = attr;
+  if (a->sync == FUSED_CLUSTER) {
+    for (blocks = 2; blocks < num_tiles; blocks <<= 1) {
+    }
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = blocks;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg->numAttrs = 1;
     int dev = 0;
     e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (!(cluster_done.load(std::memory_order_acquire) & (1ull << (dev & 63)))) {
+    const uint64_t bit = 1ull << (dev & 63);
+    if (blocks > 8 && !(state.cluster_done.load(std::memory_order_acquire) & bit)) {
       e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
       if (e != cudaSuccess) return e;
-      cluster_done.fetch_or(1ull << (dev & 63), std::memory_order_acq_rel);
+      state.cluster_done.fetch_or(bit, std::memory_order_acq_rel);
     }
+  } else if (a->sync == FUSED_GRID) {
+    attr->id = cudaLaunchAttributeCooperative;
+    attr->val.cooperative = 1;
+    cfg->numAttrs = 1;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(C::THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  if (a.sync == FUSED_CLUSTER) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = blocks;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.numAttrs = 1;
-  } else if (a.sync == FUSED_GRID) {
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.numAttrs = 1;
-  }
-  cfg.attrs = attr;
-  e = cudaLaunchKernelEx(&cfg, kern, kin, vin, kout, vout, n, a, params, reinterpret_cast<ScratchHeader*>(scratch));
-  if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device has: not all resident
-    cudaGetLastError();
+  cfg->gridDim = dim3(blocks);
+  cfg->blockDim = dim3(C::THREADS);
+  cfg->dynamicSmemBytes = smem;
+  cfg->stream = stream;
+  *fits = true;
+  return cudaSuccess;
+}
+
+// The outcome of a one-launch kernel's launch: one refused because the device
+// offers fewer SMs than it has is not an error, the stages run instead.
+inline cudaError_t fused_launched(cudaError_t e, bool* launched) {
+  *launched = e != cudaErrorCooperativeLaunchTooLarge;
+  if (*launched) return e;
+  cudaGetLastError();
+  return cudaSuccess;
+}
+
+// Runs a whole multisplit as one launch if the rule above says so and, beyond
+// one cluster, the scratch has room for the counts as [tile][bucket] rows after
+// the matrix and status words (every caller that allocated the reported size
+// has it there: its byte per key).  *launched says whether it did.
+template <class C, class P>
+cudaError_t launch_fused(const typename C::KT* kin, const typename C::VT* vin, typename C::KT* kout, typename C::VT* vout,
+                         uint32_t n, const typename P::Params& params, unsigned char* scratch, size_t scratch_bytes,
+                         const Geometry& g, cudaStream_t stream, uint32_t* starts, bool* launched) {
+  static FusedKernelState state;
+  *launched = false;
+  if (g.num_tiles > (C::KV && P::CHEAP ? FUSED_CHEAP_PAIR_TILES : FUSED_MAX_TILES)) return cudaSuccess;
+  FusedArgs a{};
+  a.starts = starts;
+  a.matrix = reinterpret_cast<uint32_t*>(scratch + g.off_matrix);
+  const size_t rows_bytes = size_t(g.m) * 4, totals_bytes = size_t(C::B) * 4;
+  if (g.num_tiles > 1 && scratch_bytes >= g.off_buckets + rows_bytes + totals_bytes) {
+    a.rows = reinterpret_cast<uint32_t*>(scratch + g.off_buckets);
+    if (g.m > FUSED_ADD_MAX) a.totals = reinterpret_cast<uint32_t*>(scratch + g.off_buckets + rows_bytes);
+  } else if (g.num_tiles > FUSED_CLUSTER_MAX) {
     return cudaSuccess;
   }
-  *launched = true;
-  return e;
+  auto kern = fused_kernel<C, P>;
+  constexpr size_t smem = PostLayout<C, P, C::KW == 2>::BYTES;
+  constexpr size_t static_smem = 2 * C::THREADS * 4 + C::B * 4 + fused_ident_words<C, P>() * 4;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  bool fits = false;
+  const cudaError_t e =
+      fused_config<C>(kern, smem, static_smem, g.num_tiles, state, stream, &a, &cfg, attr, &fits);
+  if (e != cudaSuccess || !fits) return e;
+  return fused_launched(cudaLaunchKernelEx(&cfg, kern, kin, vin, kout, vout, n, a, params,
+                                           reinterpret_cast<ScratchHeader*>(scratch)),
+                        launched);
+}
+
+// Sorts with digits of LOGB bits and tiles of IPT keys per thread in one launch,
+// if its tiles are resident at once and there is room for the count rows (or
+// they form one cluster); *launched says whether it did.
+template <int LOGB, bool KV, int KW, int VW, int IPT>
+cudaError_t launch_fused_sort(const FusedSortCall& c, bool* launched) {
+  using C = TileCfg<LOGB, 8, IPT, KV, KW, VW>;
+  using P = FieldPolicy<KW == 1>;
+  static FusedKernelState state;
+  *launched = false;
+  const uint32_t num_tiles = uint32_t((uint64_t(c.n) + C::TILE - 1) / C::TILE);
+  if (num_tiles > FUSED_MAX_TILES) return cudaSuccess;
+  FusedArgs a{};
+  const size_t rows_bytes = size_t(num_tiles) * C::B * 4;
+  if (num_tiles > 1 && c.rows_bytes >= rows_bytes + C::B * 4) {
+    a.rows = reinterpret_cast<uint32_t*>(c.rows);
+    if (num_tiles * C::B > FUSED_ADD_MAX) a.totals = reinterpret_cast<uint32_t*>(c.rows + rows_bytes);
+  } else if (num_tiles > FUSED_CLUSTER_MAX) {
+    return cudaSuccess;
+  }
+  auto kern = fused_sort_kernel<C, P>;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  bool fits = false;
+  const cudaError_t e = fused_config<C>(kern, PostLayout<C, P, KW == 2>::BYTES, (2 * C::THREADS + C::B + 1) * 4, num_tiles, state,
+                                        c.stream, &a, &cfg, attr, &fits);
+  if (e != cudaSuccess || !fits) return e;
+  using K = typename C::KT;
+  using V = typename C::VT;
+  const FusedDigits d{c.begin_bit, c.end_bit, uint32_t(LOGB)};
+  return fused_launched(cudaLaunchKernelEx(&cfg, kern, static_cast<const K*>(c.kin), static_cast<const V*>(c.vin),
+                                           static_cast<K*>(c.kout), static_cast<V*>(c.vout), static_cast<K*>(c.tk),
+                                           static_cast<V*>(c.tv), c.n, a, d, c.hdr),
+                        launched);
 }
 
 template <class P, int LOGB, bool KV, int KW = 1, int VW = 1>
@@ -167,6 +228,12 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
   auto* status = reinterpret_cast<uint64_t*>(scratch + g.off_status);
   auto* matrix = reinterpret_cast<uint32_t*>(scratch + g.off_matrix);
 
+  if (stages == STAGE_ALL) {
+    bool launched = false;
+    const cudaError_t e =
+        launch_fused<C, P>(kin, vin, kout, vout, n, params, scratch, scratch_bytes, g, stream, starts, &launched);
+    if (e != cudaSuccess || launched) return e;
+  }
   if constexpr (KW == 2) {
     if (bucket_bytes == nullptr) return cudaErrorInvalidValue;
     if (stages & STAGE_PRESCAN) {
@@ -196,14 +263,6 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
     }
     return cudaSuccess;
   } else {
-  if constexpr (VW == 1) {
-    bool launched = false;
-    if (stages == STAGE_ALL) {
-      const cudaError_t e =
-          launch_fused<C, P>(kin, vin, kout, vout, n, params, scratch, scratch_bytes, g, stream, starts, &launched);
-      if (e != cudaSuccess || launched) return e;
-    }
-  }
   if (stages & STAGE_PRESCAN) {
     static std::atomic<int> per_sm{0};
     auto kern = prescan_kernel<C, P>;
@@ -300,10 +359,10 @@ cudaError_t run_multisplit_wide_t(const MsCallWide& c, int stages) {
   if constexpr (KW == 2)
     return launch_multisplit<DescPolicy64<KIND, LOGB>, LOGB, KV, KW, VW>(kin, vin, kout, vout, c.n, c.bp64,
                                                                            c.scratch, stages, c.stream,
-                                                                           c.bucket_bytes, 0, c.starts);
+                                                                           c.bucket_bytes, c.scratch_bytes, c.starts);
   else
     return launch_multisplit<DescPolicy<KIND, LOGB>, LOGB, KV, KW, VW>(kin, vin, kout, vout, c.n, c.bp, c.scratch,
-                                                                         stages, c.stream, c.bucket_bytes, 0, c.starts);
+                                                                         stages, c.stream, c.bucket_bytes, c.scratch_bytes, c.starts);
 }
 
 template <int KIND, int LOGB>

@@ -158,6 +158,7 @@ struct MsCallWide {
   unsigned char* scratch = nullptr;  // laid out as make_geometry(n, logb, kv, kw, vw)
   cudaStream_t stream = nullptr;
   uint8_t* bucket_bytes = nullptr;
+  size_t scratch_bytes = 0;          // bytes at scratch
   uint32_t* starts = nullptr;        // pinned host memory for 2^logb bucket starts, or null
 };
 
@@ -283,6 +284,30 @@ struct BatchQueueLaunch {
   cudaStream_t stream = nullptr;
 };
 cudaError_t run_batch_queue(const BatchQueueLaunch& c);
+
+// A stable sort by key bits [begin_bit, end_bit) in one launch (inst_sort.cu),
+// for inputs whose tiles are resident at once; tk, tv are the ping-pong
+// buffers, rows an area of rows_bytes for the blocks' counts.
+struct FusedSortCall {
+  const void* kin = nullptr;
+  const void* vin = nullptr;
+  void* kout = nullptr;
+  void* vout = nullptr;
+  void* tk = nullptr;
+  void* tv = nullptr;
+  uint32_t n = 0;
+  int key_bytes = 4;
+  int value_bytes = 0;
+  uint32_t begin_bit = 0;
+  uint32_t end_bit = 32;
+  ScratchHeader* hdr = nullptr;
+  unsigned char* rows = nullptr;
+  size_t rows_bytes = 0;
+  cudaStream_t stream = nullptr;
+};
+// Bytes of the count rows such a sort of n keys uses (0: n is too large).
+size_t fused_sort_rows_bytes(uint32_t n);
+cudaError_t run_fused_sort(const FusedSortCall& c, bool* launched);
 
 // Creates a batch plan whose every class uses `variant` (>= 0), or the tuning
 // table's choice per segment (variant < 0).
