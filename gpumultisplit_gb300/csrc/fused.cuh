@@ -247,7 +247,7 @@ __device__ __forceinline__ void stage_tile(T* dst, const T* src, uint32_t cnt) {
 // Blocks per SM the fused kernel is register-budgeted for: four (64
 // registers), fewer where 64-bit elements fill the shared memory first.
 template <class C, class P>
-constexpr int fused_blocks() {
+__host__ __device__ constexpr int fused_blocks() {
   return C::WIDE && PostLayout<C, P, C::KW == 2>::MIN_BLOCKS < 4 ? PostLayout<C, P, C::KW == 2>::MIN_BLOCKS : 4;
 }
 
@@ -306,7 +306,7 @@ __device__ __forceinline__ void fused_reset_header(ScratchHeader* hdr) {
 // Shared words of a 64-bit identifier's state (32-bit ones keep theirs in the
 // tile's layout).
 template <class C, class P>
-constexpr uint32_t fused_ident_words() {
+__host__ __device__ constexpr uint32_t fused_ident_words() {
   return C::KW == 2 ? P::SMEM_WORDS : 1u;
 }
 
@@ -338,6 +338,7 @@ template <bool CHEAP_>
 struct FieldPolicy {
   using Params = FieldParams;
   using Id = FieldId;
+  template <bool KV>
   static constexpr bool CHEAP = CHEAP_;
   static constexpr bool USES_SMEM = false;
   static constexpr uint32_t SMEM_WORDS = 1;
