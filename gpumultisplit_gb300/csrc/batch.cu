@@ -424,12 +424,7 @@ gms_status batch_create(const gms_segment* segments, uint32_t count, int variant
     d.kout = sg.d_key_out;
     d.vout = sg.d_value_out;
     d.n = sg.n;
-    d.bp.shift = sg.desc.shift;
-    d.bp.param = sg.desc.param;
-    d.bp.lower = sg.desc.lower;
-    d.bp.inverse_delta = sg.desc.inverse_delta;
-    d.bp.splitters = sg.desc.d_splitters;
-    d.bp.num_buckets = sg.desc.num_buckets;
+    d.bp = to_params(sg.desc);
     if (variant < 0 && sg.n > 0 && sg.n <= kWarpSegMax) {
       // One warp multisplits the whole segment; its bucket starts get matrix
       // entries after every scan group (assigned below).
@@ -470,7 +465,7 @@ gms_status batch_create(const gms_segment* segments, uint32_t count, int variant
     d.base = uint32_t(group_n);
     d.matrix_off = uint32_t(matrix_total);
     d.bytes_off = 0;
-    if (kind_keeps_bucket_bytes(kind)) {  // one bucket byte per key, 16-byte aligned per segment
+    if (kind_keeps_bucket_bytes(kind, kv)) {  // one bucket byte per key, 16-byte aligned per segment
       d.bytes_off = byte_total;
       byte_total += (uint64_t(sg.n) + 15) & ~uint64_t(15);
     }

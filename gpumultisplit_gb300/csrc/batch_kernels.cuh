@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(C::THREADS) batch_prescan_kernel(const SegDesc
                                                                    uint32_t* __restrict__ matrix,
                                                                    uint8_t* __restrict__ byte_area) {
   using P = DescPolicy<KIND, C::LOGB>;
-  constexpr bool BYTES = !P::CHEAP;
+  constexpr bool BYTES = !P::template CHEAP<C::KV>;
   using Counter = KeyCounter<C::LOGB, typename P::Id>;
   __shared__ uint32_t s_hist[Counter::smem_words(C::WARPS)];
   __shared__ uint32_t s_split[P::SMEM_WORDS];
@@ -87,17 +87,19 @@ __global__ void __launch_bounds__(C::THREADS) batch_prescan_kernel(const SegDesc
 // prescan stored.
 template <class C, int KIND>
 __global__ void __launch_bounds__(C::THREADS,
-                                  (PostLayout<C, DescPolicy<KIND, C::LOGB>, !DescPolicy<KIND, C::LOGB>::CHEAP>::MIN_BLOCKS))
+                                  (PostLayout<C, DescPolicy<KIND, C::LOGB>,
+                                              !DescPolicy<KIND, C::LOGB>::template CHEAP<C::KV>>::MIN_BLOCKS))
     batch_postscan_kernel(const SegDesc* __restrict__ segs, const uint2* __restrict__ tile_map,
                           const uint32_t* __restrict__ matrix, ScratchHeader* hdr, const uint8_t* byte_area) {
   using P = DescPolicy<KIND, C::LOGB>;
+  constexpr bool CHEAP = P::template CHEAP<C::KV>;
   extern __shared__ __align__(128) unsigned char smem[];
   const uint2 m = tile_map[blockIdx.x];
   const SegDesc& sd = segs[m.x];
   const TileJob<BucketParams> job{sd.kin, sd.vin,  sd.kout, sd.vout, sd.n,  sd.num_tiles,
                                   m.y,    matrix + sd.matrix_off, sd.base, ~0u, sd.bp, m.x,
-                                  P::CHEAP ? nullptr : byte_area + sd.bytes_off};
-  postscan_job<C, P, true, !P::CHEAP>(job, hdr, smem);
+                                  CHEAP ? nullptr : byte_area + sd.bytes_off};
+  postscan_job<C, P, true, !CHEAP>(job, hdr, smem);
 }
 
 // ------------------------------------------------ one warp per segment

@@ -52,17 +52,6 @@ gms_status check_desc(const gms_bucket_desc* d, int* logb) {
   }
 }
 
-BucketParams to_params(const gms_bucket_desc* d) {
-  BucketParams p;
-  p.shift = d->shift;
-  p.param = d->param;
-  p.lower = d->lower;
-  p.inverse_delta = d->inverse_delta;
-  p.splitters = d->d_splitters;
-  p.num_buckets = d->num_buckets;
-  return p;
-}
-
 cudaError_t dispatch(int kind, const MsCall& c, int stages) {
   switch (kind) {
     case KIND_DELTA: return run_multisplit<KIND_DELTA>(c, stages);
@@ -147,14 +136,14 @@ gms_status multisplit_impl(const uint32_t* kin, const uint32_t* vin, uint32_t* k
   c.n = n;
   c.logb = logb;
   c.kv = kv;
-  c.bp = to_params(desc);
+  c.bp = to_params(*desc);
   c.scratch = static_cast<unsigned char*>(scratch);
   c.stream = stream;
   c.scratch_bytes = scratch_bytes;
   c.starts = starts;
   // Costly identifiers are evaluated once when the scratch has room for a
   // bucket byte per key (the prescan stores them, the postscan reads them).
-  if (kind_keeps_bucket_bytes(desc->kind) && scratch_bytes >= g.bytes_full) c.bucket_bytes = c.scratch + g.off_buckets;
+  if (kind_keeps_bucket_bytes(desc->kind, kv) && scratch_bytes >= g.bytes_full) c.bucket_bytes = c.scratch + g.off_buckets;
   return cuda_status(dispatch(desc->kind, c, stages));
 }
 
@@ -497,7 +486,7 @@ gms_status multisplit_big_impl(const uint32_t* kin, const uint32_t* vin, uint32_
   auto* base = static_cast<unsigned char*>(scratch);
   auto* tk = reinterpret_cast<uint32_t*>(base + L.off_keys);
   auto* tv = kv ? reinterpret_cast<uint32_t*>(base + L.off_vals) : nullptr;
-  const BucketParams bp = to_params(desc);
+  const BucketParams bp = to_params(*desc);
   for (int pass = 0; pass < 2; ++pass) {
     DigitPass c;
     c.kin = pass == 0 ? kin : tk;
@@ -648,8 +637,8 @@ gms_status multisplit_wide_impl(const void* kin, const void* vin, void* kout, vo
     c.bp64 = to_params64(desc);
     c.bucket_bytes = c.scratch + g.off_buckets;
   } else {
-    c.bp = to_params(&d32);
-    if (kind_keeps_bucket_bytes(desc->kind) && scratch_bytes >= g.bytes_full) c.bucket_bytes = c.scratch + g.off_buckets;
+    c.bp = to_params(d32);
+    if (kind_keeps_bucket_bytes(desc->kind, kv) && scratch_bytes >= g.bytes_full) c.bucket_bytes = c.scratch + g.off_buckets;
   }
   return cuda_status(dispatch_wide(desc->kind, c, STAGE_ALL));
 }
@@ -967,7 +956,7 @@ gms_status gms_histogram(const uint32_t* d_key_in, uint32_t n, const gms_bucket_
     if (d_hist == nullptr) return GMS_ERROR_INVALID_VALUE;
     if (n == 0) return GMS_SUCCESS;
     if (d_key_in == nullptr) return GMS_ERROR_INVALID_VALUE;
-    return cuda_status(dispatch_big_histogram(desc->kind, d_key_in, n, to_params(desc),
+    return cuda_status(dispatch_big_histogram(desc->kind, d_key_in, n, to_params(*desc),
                                               reinterpret_cast<uint32_t*>(d_hist), stream));
   }
   int logb = 0;
@@ -976,7 +965,7 @@ gms_status gms_histogram(const uint32_t* d_key_in, uint32_t n, const gms_bucket_
   if (d_hist == nullptr) return GMS_ERROR_INVALID_VALUE;
   if (n == 0) return GMS_SUCCESS;
   if (d_key_in == nullptr) return GMS_ERROR_INVALID_VALUE;
-  return cuda_status(dispatch_hist(desc->kind, d_key_in, n, logb, to_params(desc), d_hist, stream));
+  return cuda_status(dispatch_hist(desc->kind, d_key_in, n, logb, to_params(*desc), d_hist, stream));
 }
 
 gms_status gms_histogram_even(const uint32_t* d_key_in, uint32_t n, int32_t* d_hist, uint32_t num_bins,

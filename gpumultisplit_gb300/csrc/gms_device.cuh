@@ -211,6 +211,28 @@ enum BucketKind : int {
   NUM_KINDS = 6
 };
 
+// Division by a number known when the call is made, as one multiply-high, an
+// add and two shifts (Granlund and Montgomery, "Division by invariant integers
+// using multiplication", PLDI 1994, figure 4.1): with l = ceil(log2 d) and
+// mul = floor(2^32 (2^l - d) / d) + 1, n / d = (t + ((n - t) >> min(l, 1))) >>
+// max(l - 1, 0) for t = mulhi(mul, n), for every 32-bit n.
+struct Reciprocal {
+  uint32_t mul;
+  uint32_t shifts;  // min(l, 1) | max(l - 1, 0) << 8
+};
+
+inline Reciprocal reciprocal_of(uint32_t d) {  // d >= 1
+  uint32_t l = 0;
+  while (l < 32 && (uint64_t(1) << l) < d) ++l;
+  const uint64_t mul = ((((uint64_t(1) << l) - d) << 32) / d) + 1;
+  return Reciprocal{uint32_t(mul), (l < 1 ? l : 1u) | ((l > 1 ? l - 1 : 0u) << 8)};
+}
+
+__device__ __forceinline__ uint32_t divide(uint32_t n, const Reciprocal& r) {
+  const uint32_t t = __umulhi(r.mul, n);
+  return (t + ((n - t) >> (r.shifts & 1u))) >> (r.shifts >> 8);
+}
+
 // B = num_buckets may be any count in [2, 256]; the kernels run with
 // 2^LOGB >= B buckets, the ones from B up staying empty.
 struct BucketParams {
@@ -220,9 +242,20 @@ struct BucketParams {
   float inverse_delta;
   const uint32_t* splitters;  // RANGE only (device memory, B entries)
   uint32_t num_buckets;       // B
+  Reciprocal by_param;        // DIV: of param
+  Reciprocal by_buckets;      // of num_buckets
 };
 
-// v modulo b (b >= 2): a mask for powers of two, a division otherwise.
+// v modulo the bucket count: a mask for powers of two; else a quotient is rarely
+// past the buckets, so the division is skipped unless a lane needs it.
+__device__ __forceinline__ uint32_t reduce_bucket(uint32_t v, const BucketParams& p) {
+  const uint32_t b = p.num_buckets;
+  if ((b & (b - 1)) == 0) return v & (b - 1);
+  if (v >= b) v -= divide(v, p.by_buckets) * b;
+  return v;
+}
+
+// v modulo b (b >= 2): a mask for powers of two, a division otherwise (64-bit identifiers).
 __device__ __forceinline__ uint32_t reduce_mod(uint32_t v, uint32_t b) {
   return (b & (b - 1)) == 0 ? (v & (b - 1)) : (v % b);
 }
@@ -258,7 +291,7 @@ struct Identifier {
       // of the key when B = 2^LOGB).
       return __umulhi(key, p.num_buckets);
     } else if constexpr (KIND == KIND_DIV) {
-      return reduce_mod(key / p.param, p.num_buckets);
+      return reduce_bucket(divide(key, p.by_param), p);
     } else if constexpr (KIND == KIND_BITS) {
       return (key >> p.shift) & (B - 1);
     } else if constexpr (KIND == KIND_RANGE) {
@@ -301,7 +334,7 @@ struct Identifier {
       return (key & p.param) ? 1u : 0u;
     } else {  // KIND_EVEN_FLOAT
       const float x = __fmul_rn(__uint2float_rn(key - p.lower), p.inverse_delta);
-      return reduce_mod(__float2uint_rz(x), p.num_buckets);
+      return reduce_bucket(__float2uint_rz(x), p);
     }
   }
 };
@@ -348,6 +381,18 @@ __device__ __forceinline__ void prepare_identifier(uint32_t* s_split, const Buck
   }
 }
 
+// Whether an identifier kind is evaluated once, in the prescan, which keeps a
+// byte per key for the postscan, instead of in both: the splitter search
+// always, and key-only division and even-float binning.  Pairs are bound by
+// their values' traffic as well, and there the byte costs more than evaluating
+// these again.  At 2^28, ms, byte / evaluated twice: division into 32 buckets
+// keys 0.850 / 0.931, pairs 1.072 / 1.058; into 256 buckets keys 1.268 / 1.304,
+// pairs 1.489 / 1.424; even-float pairs 32 buckets 1.071 / 0.977, 256 buckets
+// 1.489 / 1.419.
+__host__ __device__ constexpr bool kind_keeps_bucket_bytes(int kind, bool kv) {
+  return kind == KIND_RANGE || (!kv && (kind == KIND_DIV || kind == KIND_EVEN_FLOAT));
+}
+
 // Identifier policies: what the kernels need to know about a bucket
 // identifier.  DescPolicy covers the precompiled descriptor kinds; the drop-in
 // C++ headers use FunctorPolicy to instantiate the same kernels with any
@@ -356,7 +401,8 @@ template <int KIND, int LOGB>
 struct DescPolicy {
   using Params = BucketParams;
   using Id = Identifier<KIND, LOGB>;
-  static constexpr bool CHEAP = KIND == KIND_DELTA || KIND == KIND_BITS || KIND == KIND_MASK;
+  template <bool KV>
+  static constexpr bool CHEAP = !kind_keeps_bucket_bytes(KIND, KV);
   static constexpr bool USES_SMEM = KIND == KIND_RANGE;
   static constexpr uint32_t SMEM_WORDS = identifier_smem_words<KIND, LOGB>();
   __device__ __forceinline__ static void prepare(uint32_t* s, const Params& p) { prepare_identifier<KIND, LOGB>(s, p); }
@@ -463,6 +509,7 @@ template <int KIND, int LOGB>
 struct DescPolicy64 {
   using Params = BucketParams64;
   using Id = Identifier64<KIND, LOGB>;
+  template <bool KV>
   static constexpr bool CHEAP = false;  // 64-bit keys always keep their buckets as bytes
   static constexpr bool USES_SMEM = KIND == KIND_RANGE;
   static constexpr uint32_t SMEM_WORDS = identifier64_smem_words<KIND, LOGB>();
@@ -503,7 +550,7 @@ __device__ __forceinline__ uint32_t big_bucket_id(uint32_t key, const BucketPara
   if constexpr (KIND == KIND_DELTA) {
     return __umulhi(key, B);
   } else if constexpr (KIND == KIND_DIV) {
-    return reduce_mod(key / p.param, B);
+    return reduce_bucket(divide(key, p.by_param), p);
   } else if constexpr (KIND == KIND_BITS) {
     return (key >> p.shift) & (B - 1);
   } else if constexpr (KIND == KIND_RANGE) {
@@ -521,7 +568,7 @@ __device__ __forceinline__ uint32_t big_bucket_id(uint32_t key, const BucketPara
     return (key & p.param) ? 1u : 0u;
   } else {  // KIND_EVEN_FLOAT
     const float x = __fmul_rn(__uint2float_rn(key - p.lower), p.inverse_delta);
-    return reduce_mod(__float2uint_rz(x), B);
+    return reduce_bucket(__float2uint_rz(x), p);
   }
 }
 
@@ -569,6 +616,7 @@ template <int KIND, int LOGB>
 struct DigitPolicy {
   using Params = BucketParamsBig;
   using Id = DigitId<KIND, LOGB>;
+  template <bool KV>
   static constexpr bool CHEAP = false;
   static constexpr bool USES_SMEM = KIND == KIND_RANGE;
   static constexpr uint32_t SMEM_WORDS = big_identifier_smem_words<KIND>();
@@ -586,6 +634,7 @@ struct GivenBytesId {
 struct GivenBytesPolicy {
   using Params = BucketParamsBig;
   using Id = GivenBytesId;
+  template <bool KV>
   static constexpr bool CHEAP = false;
   static constexpr bool USES_SMEM = false;
   static constexpr uint32_t SMEM_WORDS = 1;
@@ -607,6 +656,7 @@ template <class F, int LOGB>
 struct FunctorPolicy {
   using Params = F;
   using Id = FunctorId<F, LOGB>;
+  template <bool KV>
   static constexpr bool CHEAP = false;  // cost unknown: buckets are computed once per key and kept
   static constexpr bool USES_SMEM = false;
   static constexpr uint32_t SMEM_WORDS = 1;

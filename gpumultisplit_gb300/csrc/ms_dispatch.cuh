@@ -154,7 +154,7 @@ cudaError_t launch_fused(const typename C::KT* kin, const typename C::VT* vin, t
                          const Geometry& g, cudaStream_t stream, uint32_t* starts, bool* launched) {
   static FusedKernelState state;
   *launched = false;
-  if (g.num_tiles > (C::KV && P::CHEAP ? FUSED_CHEAP_PAIR_TILES : FUSED_MAX_TILES)) return cudaSuccess;
+  if (g.num_tiles > (C::KV && P::template CHEAP<true> ? FUSED_CHEAP_PAIR_TILES : FUSED_MAX_TILES)) return cudaSuccess;
   FusedArgs a{};
   a.starts = starts;
   a.matrix = reinterpret_cast<uint32_t*>(scratch + g.off_matrix);
@@ -219,7 +219,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
                               uint32_t n, const typename P::Params& params, unsigned char* scratch, int stages,
                               cudaStream_t stream, uint8_t* bucket_bytes = nullptr, size_t scratch_bytes = 0,
                               uint32_t* starts = nullptr) {
-  if constexpr (P::CHEAP) bucket_bytes = nullptr;
+  if constexpr (P::template CHEAP<KV>) bucket_bytes = nullptr;
   using S = TileShape<LOGB, KV, KW, VW>;
   using C = TileCfg<LOGB, S::WARPS, S::IPT, KV, KW, VW>;
   const Geometry g = make_geometry(n, LOGB, KV, KW, VW);
@@ -276,7 +276,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
     cudaError_t e = run_scan(matrix, g.m, status, hdr, stream);
     if (e != cudaSuccess) return e;
   }
-  if constexpr (!P::CHEAP) {
+  if constexpr (!P::template CHEAP<KV>) {
     if ((stages & STAGE_POSTSCAN) && bucket_bytes != nullptr) {
       // Buckets from the prescan: no identifier in the postscan at all.
       static std::atomic<uint64_t> smem_done{0};
@@ -435,7 +435,7 @@ cudaError_t run_batch_class_t(const BatchClassLaunch& c, int stage) {
     }
     static std::atomic<uint64_t> smem_done{0};
     using P = DescPolicy<KIND, LOGB>;
-    constexpr size_t smem = PostLayout<C, P, !P::CHEAP>::BYTES;
+    constexpr size_t smem = PostLayout<C, P, !P::template CHEAP<KV>>::BYTES;
     auto kern = batch_postscan_kernel<C, KIND>;
     cudaError_t e = ensure_smem_limit(kern, smem, smem_done);
     if (e != cudaSuccess) return e;

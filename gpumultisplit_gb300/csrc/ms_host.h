@@ -111,10 +111,18 @@ inline Geometry make_geometry(uint32_t n, int logb, bool kv, int kw = 1, int vw 
   return g;
 }
 
-// Identifier kinds costly enough to evaluate once (in the prescan) and keep
-// as one byte per key for the postscan.
-inline bool kind_keeps_bucket_bytes(int kind) {
-  return kind == KIND_RANGE || kind == KIND_DIV || kind == KIND_EVEN_FLOAT;
+// The device form of a 32-bit descriptor.
+inline BucketParams to_params(const gms_bucket_desc& d) {
+  BucketParams p;
+  p.shift = d.shift;
+  p.param = d.param;
+  p.lower = d.lower;
+  p.inverse_delta = d.inverse_delta;
+  p.splitters = d.d_splitters;
+  p.num_buckets = d.num_buckets;
+  p.by_param = reciprocal_of(d.param != 0 ? d.param : 1u);
+  p.by_buckets = reciprocal_of(d.num_buckets != 0 ? d.num_buckets : 1u);
+  return p;
 }
 
 enum Stage : int { STAGE_PRESCAN = 1, STAGE_SCAN = 2, STAGE_POSTSCAN = 4, STAGE_ALL = 7 };

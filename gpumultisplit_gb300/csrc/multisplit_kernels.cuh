@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(C::THREADS) prescan_kernel(const uint32_t* __r
     if (tid < C::B) s_cnt[tid * G + g] = total;
     if (g == G - 1 || tile + 1 == last) flush(tile - g);
   };
-  if constexpr (!P::CHEAP) {
+  if constexpr (!P::template CHEAP<C::KV>) {
     if (bucket_bytes != nullptr) {
       count_tiles<C::THREADS, C::IPT, true>(keys, n, first, 1u, counter, done, bucket_bytes, last);
       return;
@@ -418,8 +418,8 @@ enum ReorderMode { R_KEYS = 0, R_INDEX16 = 1, R_KEYS_B = 2, R_INDEX16_B = 3 };
 
 template <class C, class P, bool GIVEN = false>
 struct PostLayout {
-  static constexpr bool CHEAP = P::CHEAP;
-  static_assert(!GIVEN || !P::CHEAP, "given bucket bytes are only used for costly identifiers");
+  static constexpr bool CHEAP = P::template CHEAP<C::KV>;
+  static_assert(!GIVEN || !P::template CHEAP<C::KV>, "given bucket bytes are only used for costly identifiers");
   static_assert(C::KW == 1 || GIVEN, "64-bit keys take their buckets from the prescan's bytes");
   // Keys are reordered through a 16-bit index whenever values come along or
   // keys are 64 bits wide (a sorted copy of the keys would take more room).
