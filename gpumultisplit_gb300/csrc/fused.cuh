@@ -274,10 +274,9 @@ __device__ __forceinline__ void fused_tile(const typename C::KT* kin, const type
   if constexpr (C::KV) stage_tile<C::THREADS, C::IPT>(reinterpret_cast<VT*>(smem + L::OFF_V), vin + base, cnt);
   uint32_t* s_state = GIVEN ? s_ident : reinterpret_cast<uint32_t*>(smem + L::OFF_SPLIT);
   P::prepare(s_state, bp);
-  if constexpr (C::LOGB > 5) {
-    constexpr uint32_t WORDS = L::SUBWARPS * C::WB * C::WS * sizeof(typename L::WhT) / 4;
+  if constexpr (C::ATOMIC) {
     uint32_t* s_wh = reinterpret_cast<uint32_t*>(smem + L::OFF_WH);
-    for (uint32_t i = tid; i < WORDS; i += C::THREADS) s_wh[i] = 0u;
+    for (uint32_t i = tid; i < C::WARPS * C::WB; i += C::THREADS) s_wh[i] = 0u;
   }
   __syncthreads();
   if constexpr (GIVEN) {

@@ -19,18 +19,6 @@
 
 #include "gms_device.cuh"
 
-// How a warp finds, for B > 32, the lanes holding the same bucket as each lane
-// (its peer mask) in one 32-key slot:
-//   0  log2(B) bit-plane ballots (logic pipe);
-//   1  match.any (one instruction on its own pipe, but about 1.6x slower here);
-//   2  a shared-memory atomicOr of each lane's bit into a per-warp bitmap
-//      indexed by bucket, then one load (OR is order-independent, so the mask
-//      is deterministic); it trades logic work for shared-memory traffic and
-//      measured about 7% slower.
-#ifndef GMS_PEERS_MODE
-#define GMS_PEERS_MODE 0
-#endif
-
 // Threads per SM the key-only postscan's register budget is sized for: six
 // 256-thread blocks (40 registers) measured 3-5% faster than four (64) at
 // B <= 32 and equal above.
@@ -41,13 +29,6 @@
 // blocks gained 2% at B = 64 and lost 2% at B = 256; six spilled and lost more).
 #ifndef GMS_PAIRS_RESIDENT_THREADS
 #define GMS_PAIRS_RESIDENT_THREADS 1024
-#endif
-// Independent rank chains per warp at 65-128 buckets (1 or 2).  Two measured
-// 1.7 % faster there (1.178 against 1.198 ms for 2^28 pairs, and the 7-bit
-// sorts' passes 1.2 % faster); at 256 buckets the doubled count table and
-// tile scan made them 2.7 % slower, and at 64 they were equal.
-#ifndef GMS_RANK_CHAINS
-#define GMS_RANK_CHAINS 2
 #endif
 
 namespace gms {
@@ -70,9 +51,11 @@ struct TileCfg {
   using VT = std::conditional_t<VW_ == 2, uint64_t, uint32_t>;
   static_assert((KW_ == 1 || KW_ == 2) && (VW_ == 1 || VW_ == 2), "elements are 32 or 64 bits");
   static constexpr uint32_t WB = B < 32 ? 32 : B;  // row width of the per-warp count table
-  // Words per count-table entry: {peer bitmap, count} pairs when the bitmap
-  // peer search is used (B > 32), else the count alone.
-  static constexpr uint32_t WS = (LOGB_ > 5 && GMS_PEERS_MODE == 2) ? 2 : 1;
+  // Ranks by shared-memory atomics (postscan_tile); by ballots at the smallest
+  // bucket counts, where few ballots suffice and many lanes meet in a counter.
+  // At 2^28, ballots / atomics: pairs 16 buckets 0.893 / 0.866 ms, 32 buckets
+  // 0.955 / 0.867; keys 16 buckets 0.694 / 0.725, 32 buckets 0.770 / 0.712.
+  static constexpr bool ATOMIC = LOGB_ >= (KV_ ? 4 : 5);
 
   static_assert(IPT % 4 == 0, "IPT must be a multiple of 4 (16-byte vector loads)");
   static_assert(TILE <= 65536, "in-tile positions are packed into 16 bits");
@@ -412,8 +395,10 @@ __global__ void __launch_bounds__(C::THREADS) prescan64_kernel(const uint64_t* _
 //   R_KEYS_B,    the same plus the key's bucket as one byte, for identifiers
 //   R_INDEX16_B  that are costly to recompute (RANGE, DIV, EVEN_FLOAT, user
 //                functors).
-// The per-warp count table holds 16-bit entries (a warp counts at most
-// 32 * IPT keys and a tile holds at most 2^16), except in the bitmap peer mode.
+// With ranks by atomics the source index is always kept (R_INDEX16, R_INDEX16_B):
+// it shows whether the ranks kept the input order.  The per-warp count table
+// then holds 32-bit entries, which the atomics need, else 16-bit ones (a warp
+// counts at most 32 * IPT keys and a tile holds at most 2^16).
 enum ReorderMode { R_KEYS = 0, R_INDEX16 = 1, R_KEYS_B = 2, R_INDEX16_B = 3 };
 
 template <class C, class P, bool GIVEN = false>
@@ -421,27 +406,21 @@ struct PostLayout {
   static constexpr bool CHEAP = P::template CHEAP<C::KV>;
   static_assert(!GIVEN || !P::template CHEAP<C::KV>, "given bucket bytes are only used for costly identifiers");
   static_assert(C::KW == 1 || GIVEN, "64-bit keys take their buckets from the prescan's bytes");
-  // Keys are reordered through a 16-bit index whenever values come along or
-  // keys are 64 bits wide (a sorted copy of the keys would take more room).
+  // Keys are reordered through a 16-bit index whenever values come along, keys
+  // are 64 bits wide (a sorted copy of the keys would take more room) or the
+  // ranks come from atomics.
   static constexpr int MODE =
-      (C::KV || C::KW == 2) ? (CHEAP ? R_INDEX16 : R_INDEX16_B) : (CHEAP ? R_KEYS : R_KEYS_B);
+      (C::KV || C::KW == 2 || C::ATOMIC) ? (CHEAP ? R_INDEX16 : R_INDEX16_B) : (CHEAP ? R_KEYS : R_KEYS_B);
   static constexpr bool INDEXED = MODE == R_INDEX16 || MODE == R_INDEX16_B;
   static constexpr bool BUCKET_BYTES = MODE == R_KEYS_B || MODE == R_INDEX16_B;
-  using WhT = std::conditional_t<C::WS == 2, uint32_t, uint16_t>;
+  using WhT = std::conditional_t<C::ATOMIC, uint32_t, uint16_t>;
   static constexpr size_t OFF_K = 0;
   static constexpr size_t OFF_V = OFF_K + size_t(C::TILE) * sizeof(typename C::KT);
   static constexpr size_t OFF_R = OFF_V + (C::KV ? size_t(C::TILE) * sizeof(typename C::VT) : 0);
   static constexpr size_t R_BYTES = size_t(C::TILE) * (INDEXED ? 2 : 4);
   static constexpr size_t OFF_RB = OFF_R + R_BYTES;  // bucket bytes
   static constexpr size_t OFF_WH = (OFF_RB + (BUCKET_BYTES ? C::TILE : 0) + 15) & ~size_t(15);
-  // At 65-128 buckets a warp ranks its slots in CHAINS independent runs
-  // (slots [c*IPT/CHAINS, (c+1)*IPT/CHAINS) against count table c), so the
-  // table's read-modify-write chains of the runs interleave.  Sub-warp
-  // w*CHAINS + c holds the keys of run c of warp w, in input order.
-  static constexpr int CHAINS =
-      (C::LOGB == 7 && C::WS == 1 && GMS_PEERS_MODE == 0 && C::IPT % GMS_RANK_CHAINS == 0) ? GMS_RANK_CHAINS : 1;
-  static constexpr int SUBWARPS = C::WARPS * CHAINS;
-  static constexpr size_t OFF_DELTA = (OFF_WH + size_t(SUBWARPS) * C::WB * C::WS * sizeof(WhT) + 15) & ~size_t(15);
+  static constexpr size_t OFF_DELTA = (OFF_WH + size_t(C::WARPS) * C::WB * sizeof(WhT) + 15) & ~size_t(15);
   static constexpr size_t OFF_SPLIT = OFF_DELTA + C::B * 4;
   // With bucket bytes from the prescan the identifier is never evaluated, so
   // it needs no shared area.
@@ -459,6 +438,17 @@ struct PostLayout {
       C::WIDE ? (SMEM_BLOCKS < THREAD_BLOCKS ? (SMEM_BLOCKS > 0 ? SMEM_BLOCKS : 1) : THREAD_BLOCKS) : THREAD_BLOCKS;
 };
 
+// Puts the source indices of one bucket's run into ascending order (the input's
+// order).  An insertion sort: runs that are nearly in order cost one pass.
+__host__ __device__ inline void sort_run(uint16_t* run, uint32_t n) {
+  for (uint32_t i = 1; i < n; ++i) {
+    const uint16_t v = run[i];
+    uint32_t k = i;
+    for (; k > 0 && run[k - 1] > v; --k) run[k] = run[k - 1];
+    run[k] = v;
+  }
+}
+
 // Peer mask (lanes of this warp whose key in this slot has bucket b) from
 // log2(B) bit-plane ballots: lanes agree on bit i iff ballot_i ^ own_i is set,
 // with own_i = 0 or ~0 by this lane's bit i.
@@ -473,6 +463,12 @@ __device__ __forceinline__ uint32_t peers_by_ballot(uint32_t b) {
   }
   return peers;
 }
+
+// Lanes of a warp's first slot in one bucket from which on the warp treats its
+// most frequent buckets apart (with few buckets a crowd is no sign of skew).
+// 33.5 M Zipf pairs into 16 buckets took 130 us at 8 lanes and 122 at 12; keys
+// in four of 128 buckets 167 at 8 and 209 at 12.
+__host__ __device__ constexpr uint32_t rank_crowd(int logb) { return logb <= 5 ? 12u : 8u; }
 
 // Where a tile's global bucket offsets come from.  Thread b < B holds the
 // source for bucket b: aggregate() is called once the tile's count of bucket b
@@ -524,7 +520,6 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
   constexpr int LOGB = C::LOGB;
   constexpr int IPT = C::IPT;
   constexpr uint32_t WB = C::WB;
-  constexpr uint32_t WS = C::WS;
   KT* s_k = reinterpret_cast<KT*>(smem + L::OFF_K);
   VT* s_v = reinterpret_cast<VT*>(smem + L::OFF_V);
   uint32_t* s_r = reinterpret_cast<uint32_t*>(smem + L::OFF_R);
@@ -550,7 +545,77 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
   uint32_t packed[IPT];  // (bucket << 16) | rank among same-bucket keys of this warp
   const uint32_t wbase = warp * (IPT * 32u);
   const uint32_t lt = lanemask_lt();
-  if constexpr (LOGB <= 5) {
+  if constexpr (C::ATOMIC) {
+    // A key's rank is what an atomic add on its bucket's counter returns.  The
+    // adds of a warp do not depend on one another, so all its slots are in
+    // flight at once, where ballots took 4 LOGB instructions a slot and a
+    // read-modify-write of the count table that each slot waited for: ranking
+    // 2^28 keys alone took 0.68 ms with ballots and takes 0.18 at 256 buckets
+    // (0.62 and 0.17 at 128).  Lanes of one slot that meet in a bucket are
+    // served in lane order on this chip, but nothing promises it: phase 4
+    // checks every tile's order and repairs a run that is out of order.
+    // Postscan of 2^25 elements, ballots / atomics: keys 128 buckets 112 / 88
+    // us, 256 125 / 104; pairs 128 buckets 130 / 111, 256 148 / 143.
+    uint32_t* wh = reinterpret_cast<uint32_t*>(s_wh) + warp * WB;
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) packed[j] = bucket_at(wbase + uint32_t(j) * 32u + lane) << 16;
+    // Lanes that meet in a counter are served one after another, so a warp
+    // whose first slot is crowded takes its two most frequent buckets by one
+    // ballot each, their counts in registers; if a third is crowded too, all
+    // buckets go by ballots.
+    const uint32_t b0 = packed[0] >> 16;
+    const uint32_t peers0 =
+        FULL ? peers_by_ballot<LOGB>(b0) : peers_by_ballot<LOGB>(b0) & __ballot_sync(~0u, wbase + lane < cnt);
+    const uint32_t crowd = (uint32_t(__popc(peers0)) << 16) | b0;
+    const uint32_t most = __reduce_max_sync(~0u, crowd);
+    if ((most >> 16) < rank_crowd(LOGB)) {
+#pragma unroll
+      for (int j = 0; j < IPT; ++j) {
+        const uint32_t pos = wbase + uint32_t(j) * 32u + lane;
+        if (FULL || pos < cnt) packed[j] |= atomicAdd(wh + (packed[j] >> 16), 1u);
+      }
+    } else {
+      const uint32_t d1 = most & 0xFFFFu;
+      const uint32_t next = __reduce_max_sync(~0u, b0 == d1 ? 0u : crowd);
+      const uint32_t d2 = next != 0u ? next & 0xFFFFu : 0xFFFFu;
+      const uint32_t third = __reduce_max_sync(~0u, b0 == d1 || b0 == d2 ? 0u : crowd);
+      if ((third >> 16) < rank_crowd(LOGB)) {
+        uint32_t run1 = 0, run2 = 0;
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) {
+          const bool valid = FULL || wbase + uint32_t(j) * 32u + lane < cnt;
+          const uint32_t b = packed[j] >> 16;
+          const uint32_t m1 = __ballot_sync(~0u, valid && b == d1), m2 = __ballot_sync(~0u, valid && b == d2);
+          if (b == d1)
+            packed[j] |= run1 + __popc(m1 & lt);
+          else if (b == d2)
+            packed[j] |= run2 + __popc(m2 & lt);
+          else if (valid)
+            packed[j] |= atomicAdd(wh + b, 1u);
+          run1 += __popc(m1);
+          run2 += __popc(m2);
+        }
+        if (lane == 0) {
+          wh[d1] = run1;
+          if (d2 < B) wh[d2] = run2;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) {
+          const bool valid = FULL || wbase + uint32_t(j) * 32u + lane < cnt;
+          const uint32_t b = packed[j] >> 16;
+          uint32_t peers = peers_by_ballot<LOGB>(b);
+          if (!FULL) peers &= __ballot_sync(~0u, valid);
+          const uint32_t rank = __popc(peers & lt);
+          const uint32_t before = wh[b];
+          __syncwarp();
+          if (valid && rank == 0) wh[b] = before + __popc(peers);
+          __syncwarp();
+          packed[j] |= before + rank;
+        }
+      }
+    }
+  } else {
     // Lane l counts bucket l: its mask of lanes holding bucket l comes straight
     // from the ballots, and a key's peers and earlier count are read from the
     // lane that owns its bucket.
@@ -571,69 +636,6 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
       my_cnt += __popc(m);
     }
     if (lane < B) s_wh[warp * WB + lane] = WhT(my_cnt);
-  } else {
-    WhT* wh = s_wh + warp * WB * WS;  // entry b: count at [b*WS + WS-1], bitmap at [b*WS] when WS == 2
-    if constexpr (GMS_PEERS_MODE == 2) {
-#pragma unroll
-      for (int j = 0; j < IPT; ++j) {
-        const uint32_t pos = wbase + uint32_t(j) * 32u + lane;
-        const bool valid = FULL || pos < cnt;
-        const uint32_t b = bucket_at(pos);
-        uint32_t* e = reinterpret_cast<uint32_t*>(&wh[b * WS]);
-        if (valid) atomicOr(e, 1u << lane);
-        __syncwarp();
-        const uint2 v = *reinterpret_cast<const uint2*>(e);
-        const uint32_t rank = __popc(v.x & lt);
-        __syncwarp();
-        if (valid && rank == 0) *reinterpret_cast<uint2*>(e) = make_uint2(0u, v.y + __popc(v.x));
-        __syncwarp();
-        packed[j] = (b << 16) | (v.y + rank);
-      }
-    } else if constexpr (L::CHAINS == 2) {
-      // Slots j and j + IPT/2 step together, each against its own table.
-      constexpr int HALF = IPT / 2;
-      WhT* wa = s_wh + (warp * 2) * WB;
-      WhT* wb = wa + WB;
-#pragma unroll
-      for (int j = 0; j < HALF; ++j) {
-        const uint32_t pa = wbase + uint32_t(j) * 32u + lane, pb = pa + uint32_t(HALF) * 32u;
-        const bool va = FULL || pa < cnt, vb = FULL || pb < cnt;
-        const uint32_t ba = bucket_at(pa), bb = bucket_at(pb);
-        uint32_t qa = peers_by_ballot<LOGB>(ba), qb = peers_by_ballot<LOGB>(bb);
-        if (!FULL) {
-          qa &= __ballot_sync(~0u, va);
-          qb &= __ballot_sync(~0u, vb);
-        }
-        const uint32_t ra = __popc(qa & lt), rb = __popc(qb & lt);
-        const uint32_t xa = wa[ba], xb = wb[bb];
-        __syncwarp();
-        if (va && ra == 0) wa[ba] = WhT(xa + __popc(qa));
-        if (vb && rb == 0) wb[bb] = WhT(xb + __popc(qb));
-        __syncwarp();
-        packed[j] = (ba << 16) | (xa + ra);
-        packed[j + HALF] = (bb << 16) | (xb + rb);
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < IPT; ++j) {
-        const uint32_t pos = wbase + uint32_t(j) * 32u + lane;
-        const bool valid = FULL || pos < cnt;
-        const uint32_t b = bucket_at(pos);
-#if GMS_PEERS_MODE == 1
-        uint32_t peers = __match_any_sync(~0u, b);
-#else
-        uint32_t peers = peers_by_ballot<LOGB>(b);
-#endif
-        if (!FULL) peers &= __ballot_sync(~0u, valid);
-        const uint32_t rank = __popc(peers & lt);
-        WhT* e = &wh[b * WS + (WS - 1)];
-        const uint32_t before = *e;
-        __syncwarp();
-        if (valid && rank == 0) *e = WhT(before + __popc(peers));
-        __syncwarp();
-        packed[j] = (b << 16) | (before + rank);
-      }
-    }
   }
   __syncthreads();
 
@@ -646,13 +648,13 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
     // scan and write each count-table entry once; key-only tiles, budgeted at
     // 40 registers, write the prefixes and add the start in a second pass.
     constexpr bool PREFIX_IN_REGS = C::KV;
-    constexpr int SW = LOGB > 5 ? L::SUBWARPS : C::WARPS;  // count-table rows
+    constexpr int SW = C::WARPS;  // count-table rows
     uint32_t pre[PREFIX_IN_REGS ? SW : 1];
     uint32_t total = 0;
     if (tid < B) {
 #pragma unroll
       for (int w = 0; w < SW; ++w) {
-        WhT* c_ptr = &s_wh[(w * WB + tid) * WS + (WS - 1)];
+        WhT* c_ptr = &s_wh[w * WB + tid];
         const uint32_t c = *c_ptr;
         if constexpr (PREFIX_IN_REGS)
           pre[w] = total;
@@ -688,7 +690,7 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
       }
 #pragma unroll
       for (int w = 0; w < SW; ++w) {
-        WhT* c_ptr = &s_wh[(w * WB + tid) * WS + (WS - 1)];
+        WhT* c_ptr = &s_wh[w * WB + tid];
         if constexpr (PREFIX_IN_REGS)
           *c_ptr = WhT(pre[w] + start);
         else
@@ -706,15 +708,13 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
 
   // ---- 3. bucket-sorted in-tile order (positions are a permutation of [0, cnt))
   {
-    constexpr int CH = LOGB > 5 ? L::CHAINS : 1;
-    const WhT* wh = s_wh + warp * CH * WB * WS + (WS - 1);
+    const WhT* wh = s_wh + warp * WB;
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
       const uint32_t pos = wbase + uint32_t(j) * 32u + lane;
       if (FULL || pos < cnt) {
         const uint32_t b = packed[j] >> 16;
-        const WhT* row = wh + (j / (IPT / CH)) * WB * WS;  // the slot's chain
-        const uint32_t d = uint32_t(row[b * WS]) + (packed[j] & 0xFFFFu);
+        const uint32_t d = uint32_t(wh[b]) + (packed[j] & 0xFFFFu);
         if constexpr (L::INDEXED)
           reinterpret_cast<uint16_t*>(s_r)[d] = uint16_t(pos);
         else
@@ -747,6 +747,63 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
   static_assert(!STREAM_HINTS || (C::KW == 1 && C::VW == 1), "store hints are for 32-bit elements");
   uint64_t policy = 0;
   if constexpr (STREAM_HINTS) policy = l2_evict_first_policy();
+  // The key at in-tile position src goes to sorted position p of bucket b.
+  auto store = [&](uint32_t p, uint32_t src, const KT& key, uint32_t b) {
+    const uint32_t g = s_delta[b] + p;
+    if constexpr (STREAM_HINTS) {
+      st_global_hint(kout + g, key, policy);
+      if constexpr (C::KV) st_global_hint(vout + g, s_v[src], policy);
+    } else {
+      kout[g] = key;
+      if constexpr (C::KV) vout[g] = s_v[src];
+    }
+  };
+  if constexpr (C::ATOMIC) {
+    // Each warp walks its own stretch of the sorted order and checks, beside
+    // the stores, that (bucket, source) ascends from each position to the next.
+    // If it does not somewhere in the tile, every run is put in order and the
+    // tile is stored again.
+    uint16_t* s_idx = reinterpret_cast<uint16_t*>(s_r);
+    for (int attempt = 0; attempt < 2; ++attempt) {
+      bool late = false;
+      uint32_t before = 0;  // (bucket, source) of the position before this warp's slot, in lane 0
+      if (lane == 0 && wbase != 0 && (FULL || wbase < cnt)) {
+        const uint32_t src = s_idx[wbase - 1];
+        uint32_t b;
+        if constexpr (L::BUCKET_BYTES)
+          b = s_rb[wbase - 1];
+        else
+          b = ident(s_k[src]);
+        before = (b << 16) | src;
+      }
+#pragma unroll
+      for (int j = 0; j < IPT; ++j) {
+        const uint32_t p = wbase + uint32_t(j) * 32u + lane;
+        uint32_t at = ~0u;
+        if (FULL || p < cnt) {
+          const uint32_t src = s_idx[p];
+          const KT key = s_k[src];
+          uint32_t b;
+          if constexpr (L::BUCKET_BYTES)
+            b = s_rb[p];
+          else
+            b = ident(key);
+          at = (b << 16) | src;
+          store(p, src, key, b);
+        }
+        const uint32_t left = __shfl_sync(~0u, at, (lane + 31u) & 31u);
+        late |= (lane == 0 ? before : left) > at;
+        before = left;  // lane 0: the slot's last
+      }
+      if (!__syncthreads_or(late)) break;
+      if (tid < B) {  // s_wh[b] of warp 0 is the start of bucket b's run
+        const uint32_t first = s_wh[tid], last = tid + 1 < B ? uint32_t(s_wh[tid + 1]) : cnt;
+        sort_run(s_idx + first, last - first);
+      }
+      __syncthreads();
+    }
+    return true;
+  }
 #pragma unroll
   for (int j = 0; j < IPT; ++j) {
     const uint32_t p = uint32_t(j) * C::THREADS + tid;
@@ -764,14 +821,7 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
           b = s_rb[p];
         else
           b = ident(key);
-        const uint32_t g = s_delta[b] + p;
-        if constexpr (STREAM_HINTS) {
-          st_global_hint(kout + g, key, policy);
-          if constexpr (C::KV) st_global_hint(vout + g, s_v[src], policy);
-        } else {
-          kout[g] = key;
-          if constexpr (C::KV) vout[g] = s_v[src];
-        }
+        store(p, src, key, b);
       }
     }
   }
@@ -833,7 +883,6 @@ __device__ __forceinline__ bool postscan_job(const TileJob<typename P::Params, t
   using KT = typename C::KT;
   using VT = typename C::VT;
   constexpr uint32_t B = C::B;
-  constexpr int LOGB = C::LOGB;
   constexpr uint32_t WB = C::WB;
   KT* s_k = reinterpret_cast<KT*>(smem + L::OFF_K);
   VT* s_v = reinterpret_cast<VT*>(smem + L::OFF_V);
@@ -894,10 +943,8 @@ __device__ __forceinline__ bool postscan_job(const TileJob<typename P::Params, t
   if (bar_live) *bar_live = bulk != 0;
   auto offs = make_offsets(job, tid, B);
   if constexpr (PREPARE && !GIVEN) P::prepare(s_split, job.bp);
-  if constexpr (LOGB > 5) {
-    // the count table as 32-bit words (its byte size is a multiple of 4)
-    constexpr uint32_t WORDS = L::SUBWARPS * WB * C::WS * sizeof(typename L::WhT) / 4;
-    for (uint32_t i = tid; i < WORDS; i += C::THREADS) s_wh[i] = 0u;
+  if constexpr (C::ATOMIC) {
+    for (uint32_t i = tid; i < C::WARPS * WB; i += C::THREADS) s_wh[i] = 0u;
   }
   __syncthreads();
   if (bulk != 0) {
