@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(C::THREADS) prescan64_kernel(const uint64_t* _
 //                a small buffer keeps four tiles resident per SM;
 //   R_KEYS_B,    the same plus the key's bucket as one byte, for identifiers
 //   R_INDEX16_B  that are costly to recompute (RANGE, DIV, EVEN_FLOAT, user
-//                functors).
+//                functors); index and bucket as one word where there is room.
 // With ranks by atomics the source index is always kept (R_INDEX16, R_INDEX16_B):
 // it shows whether the ranks kept the input order.  The per-warp count table
 // then holds 32-bit entries, which the atomics need, else 16-bit ones (a warp
@@ -414,12 +414,28 @@ struct PostLayout {
   static constexpr bool INDEXED = MODE == R_INDEX16 || MODE == R_INDEX16_B;
   static constexpr bool BUCKET_BYTES = MODE == R_KEYS_B || MODE == R_INDEX16_B;
   using WhT = std::conditional_t<C::ATOMIC, uint32_t, uint16_t>;
+  // Blocks per SM the register budget is sized for (64 registers at 16 keys per thread).
+  static constexpr int RESIDENT_THREADS = C::IPT <= 8 ? 1536 : (C::KV ? GMS_PAIRS_RESIDENT_THREADS : GMS_KEYS_RESIDENT_THREADS);
+  static constexpr int THREAD_BLOCKS = RESIDENT_THREADS / C::THREADS > 0 ? RESIDENT_THREADS / C::THREADS : 1;
   static constexpr size_t OFF_K = 0;
   static constexpr size_t OFF_V = OFF_K + size_t(C::TILE) * sizeof(typename C::KT);
   static constexpr size_t OFF_R = OFF_V + (C::KV ? size_t(C::TILE) * sizeof(typename C::VT) : 0);
-  static constexpr size_t R_BYTES = size_t(C::TILE) * (INDEXED ? 2 : 4);
-  static constexpr size_t OFF_RB = OFF_R + R_BYTES;  // bucket bytes
-  static constexpr size_t OFF_WH = (OFF_RB + (BUCKET_BYTES ? C::TILE : 0) + 15) & ~size_t(15);
+  // With ranks by atomics, a kept bucket and the source index go into one
+  // 32-bit word (one scattered store instead of two) where that costs no
+  // resident block (228 KB per SM, 1 KB of it reserved per block).
+  static constexpr size_t REST = OFF_R + size_t(C::WARPS) * C::WB * sizeof(WhT) + C::B * 4 +
+                                 (GIVEN ? 0 : P::SMEM_WORDS * 4) + 256;
+  static constexpr int blocks_at(size_t per_key) {
+    const int by_smem = int((228u * 1024u) / (REST + size_t(C::TILE) * per_key + 1024u));
+    return by_smem < THREAD_BLOCKS ? by_smem : THREAD_BLOCKS;
+  }
+  static constexpr bool WORDS = C::ATOMIC && BUCKET_BYTES && blocks_at(4) >= blocks_at(3);
+  static constexpr size_t R_BYTES = size_t(C::TILE) * (INDEXED && !WORDS ? 2 : 4);
+  // Bucket bytes; under the words the staged ones lie where the words go, read
+  // in phase 1 before phase 3 writes.
+  static constexpr size_t OFF_RB = WORDS ? OFF_R : OFF_R + R_BYTES;
+  static constexpr size_t END_R = WORDS ? OFF_R + R_BYTES : OFF_RB + (BUCKET_BYTES ? C::TILE : 0);
+  static constexpr size_t OFF_WH = (END_R + 15) & ~size_t(15);
   static constexpr size_t OFF_DELTA = (OFF_WH + size_t(C::WARPS) * C::WB * sizeof(WhT) + 15) & ~size_t(15);
   static constexpr size_t OFF_SPLIT = OFF_DELTA + C::B * 4;
   // With bucket bytes from the prescan the identifier is never evaluated, so
@@ -428,11 +444,7 @@ struct PostLayout {
   static constexpr size_t OFF_FLAG = OFF_SCAN + 32 * 4;  // warp totals of the tile scan
   static constexpr size_t OFF_BAR = (OFF_FLAG + 4 + 15) & ~size_t(15);
   static constexpr size_t BYTES = OFF_BAR + 16;
-  // Blocks per SM the register budget is sized for (64 registers at 16 keys per thread).
-  static constexpr int RESIDENT_THREADS = C::IPT <= 8 ? 1536 : (C::KV ? GMS_PAIRS_RESIDENT_THREADS : GMS_KEYS_RESIDENT_THREADS);
-  static constexpr int THREAD_BLOCKS = RESIDENT_THREADS / C::THREADS > 0 ? RESIDENT_THREADS / C::THREADS : 1;
-  // With 64-bit elements shared memory bounds the blocks per SM first
-  // (228 KB per SM, 1 KB of it reserved per block).
+  // With 64-bit elements shared memory bounds the blocks per SM first.
   static constexpr int SMEM_BLOCKS = int((228u * 1024u) / (BYTES + 1024u));
   static constexpr int MIN_BLOCKS =
       C::WIDE ? (SMEM_BLOCKS < THREAD_BLOCKS ? (SMEM_BLOCKS > 0 ? SMEM_BLOCKS : 1) : THREAD_BLOCKS) : THREAD_BLOCKS;
@@ -440,9 +452,10 @@ struct PostLayout {
 
 // Puts the source indices of one bucket's run into ascending order (the input's
 // order).  An insertion sort: runs that are nearly in order cost one pass.
-__host__ __device__ inline void sort_run(uint16_t* run, uint32_t n) {
+template <class T>
+__host__ __device__ inline void sort_run(T* run, uint32_t n) {
   for (uint32_t i = 1; i < n; ++i) {
-    const uint16_t v = run[i];
+    const T v = run[i];
     uint32_t k = i;
     for (; k > 0 && run[k - 1] > v; --k) run[k] = run[k - 1];
     run[k] = v;
@@ -715,11 +728,13 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
       if (FULL || pos < cnt) {
         const uint32_t b = packed[j] >> 16;
         const uint32_t d = uint32_t(wh[b]) + (packed[j] & 0xFFFFu);
-        if constexpr (L::INDEXED)
+        if constexpr (L::WORDS)
+          s_r[d] = (b << 16) | pos;
+        else if constexpr (L::INDEXED)
           reinterpret_cast<uint16_t*>(s_r)[d] = uint16_t(pos);
         else
           s_r[d] = s_k[pos];
-        if constexpr (L::BUCKET_BYTES) s_rb[d] = uint8_t(b);
+        if constexpr (L::BUCKET_BYTES && !L::WORDS) s_rb[d] = uint8_t(b);
       }
     }
   }
@@ -763,33 +778,30 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
     // the stores, that (bucket, source) ascends from each position to the next.
     // If it does not somewhere in the tile, every run is put in order and the
     // tile is stored again.
-    uint16_t* s_idx = reinterpret_cast<uint16_t*>(s_r);
+    using IndexT = std::conditional_t<L::WORDS, uint32_t, uint16_t>;
+    IndexT* s_idx = reinterpret_cast<IndexT*>(s_r);
+    // (bucket << 16) | source of sorted position p.
+    auto entry = [&](uint32_t p) -> uint32_t {
+      const uint32_t e = s_idx[p];
+      if constexpr (L::WORDS)
+        return e;
+      else if constexpr (L::BUCKET_BYTES)
+        return (uint32_t(s_rb[p]) << 16) | e;
+      else
+        return (ident(s_k[e]) << 16) | e;
+    };
     for (int attempt = 0; attempt < 2; ++attempt) {
       bool late = false;
-      uint32_t before = 0;  // (bucket, source) of the position before this warp's slot, in lane 0
-      if (lane == 0 && wbase != 0 && (FULL || wbase < cnt)) {
-        const uint32_t src = s_idx[wbase - 1];
-        uint32_t b;
-        if constexpr (L::BUCKET_BYTES)
-          b = s_rb[wbase - 1];
-        else
-          b = ident(s_k[src]);
-        before = (b << 16) | src;
-      }
+      uint32_t before = 0;  // entry of the position before this warp's slot, in lane 0
+      if (lane == 0 && wbase != 0 && (FULL || wbase < cnt)) before = entry(wbase - 1);
 #pragma unroll
       for (int j = 0; j < IPT; ++j) {
         const uint32_t p = wbase + uint32_t(j) * 32u + lane;
         uint32_t at = ~0u;
         if (FULL || p < cnt) {
-          const uint32_t src = s_idx[p];
-          const KT key = s_k[src];
-          uint32_t b;
-          if constexpr (L::BUCKET_BYTES)
-            b = s_rb[p];
-          else
-            b = ident(key);
-          at = (b << 16) | src;
-          store(p, src, key, b);
+          at = entry(p);
+          const uint32_t src = at & 0xFFFFu;
+          store(p, src, s_k[src], at >> 16);
         }
         const uint32_t left = __shfl_sync(~0u, at, (lane + 31u) & 31u);
         late |= (lane == 0 ? before : left) > at;
