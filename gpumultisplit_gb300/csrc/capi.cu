@@ -114,7 +114,7 @@ thread_local HostStarts t_starts;
 // Shared body of the multisplit entry points (stage mask selects the kernels).
 gms_status multisplit_impl(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, uint32_t n,
                            const gms_bucket_desc* desc, bool kv, void* scratch, size_t scratch_bytes,
-                           int stages, cudaStream_t stream, uint32_t* starts = nullptr) {
+                           int stages, cudaStream_t stream, uint32_t* starts = nullptr, bool keep_matrix = true) {
   int logb = 0;
   gms_status st = check_desc(desc, &logb);
   if (st != GMS_SUCCESS) return st;
@@ -141,6 +141,7 @@ gms_status multisplit_impl(const uint32_t* kin, const uint32_t* vin, uint32_t* k
   c.stream = stream;
   c.scratch_bytes = scratch_bytes;
   c.starts = starts;
+  c.keep_matrix = keep_matrix;
   // Costly identifiers are evaluated once when the scratch has room for a
   // bucket byte per key (the prescan stores them, the postscan reads them).
   if (kind_keeps_bucket_bytes(desc->kind, kv) && scratch_bytes >= g.bytes_full) c.bucket_bytes = c.scratch + g.off_buckets;
@@ -347,7 +348,7 @@ gms_status sort_run(const uint32_t* kin, uint32_t* kout, const uint32_t* vin, ui
     d.num_buckets = sch.buckets[p];
     d.shift = sch.shift[p];
     gms_status st = multisplit_impl(ki, kv ? vi : nullptr, ko, kv ? vo : nullptr, n, &d, kv, scratch, L.ms_bytes,
-                                    STAGE_ALL, stream);
+                                    STAGE_ALL, stream, nullptr, false);
     if (st != GMS_SUCCESS) return st;
     ki = ko;
     vi = vo;
@@ -367,7 +368,8 @@ gms_status compaction_impl(const uint32_t* kin, const uint32_t* vin, uint32_t* k
                            uint32_t* h_num0, cudaStream_t stream) {
   if (desc == nullptr || desc->num_buckets != 2) return GMS_ERROR_INVALID_VALUE;
   uint32_t* starts = h_num0 != nullptr && n != 0 ? t_starts.get() : nullptr;
-  gms_status st = multisplit_impl(kin, vin, kout, vout, n, desc, kv, scratch, scratch_bytes, STAGE_ALL, stream, starts);
+  gms_status st = multisplit_impl(kin, vin, kout, vout, n, desc, kv, scratch, scratch_bytes, STAGE_ALL, stream, starts,
+                                  h_num0 != nullptr && starts == nullptr);
   if (st != GMS_SUCCESS || h_num0 == nullptr) return st;
   // Start of bucket 1 = number of bucket-0 keys (multisplit2_compaction.cuh:541-542).
   uint32_t offsets[2];
@@ -428,14 +430,14 @@ gms_status check_big_desc(const gms_bucket_desc* d) {
   }
 }
 
-cudaError_t dispatch_digit_prescan(int kind, const DigitPass& c) {
+cudaError_t dispatch_digit_prescan(int kind, const DigitPass& c, uint32_t* rows_per) {
   switch (kind) {
-    case KIND_DELTA: return run_digit_prescan_scan<KIND_DELTA>(c);
-    case KIND_DIV: return run_digit_prescan_scan<KIND_DIV>(c);
-    case KIND_BITS: return run_digit_prescan_scan<KIND_BITS>(c);
-    case KIND_RANGE: return run_digit_prescan_scan<KIND_RANGE>(c);
-    case KIND_MASK: return run_digit_prescan_scan<KIND_MASK>(c);
-    case KIND_EVEN_FLOAT: return run_digit_prescan_scan<KIND_EVEN_FLOAT>(c);
+    case KIND_DELTA: return run_digit_prescan_scan<KIND_DELTA>(c, rows_per);
+    case KIND_DIV: return run_digit_prescan_scan<KIND_DIV>(c, rows_per);
+    case KIND_BITS: return run_digit_prescan_scan<KIND_BITS>(c, rows_per);
+    case KIND_RANGE: return run_digit_prescan_scan<KIND_RANGE>(c, rows_per);
+    case KIND_MASK: return run_digit_prescan_scan<KIND_MASK>(c, rows_per);
+    case KIND_EVEN_FLOAT: return run_digit_prescan_scan<KIND_EVEN_FLOAT>(c, rows_per);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -501,7 +503,7 @@ gms_status multisplit_big_impl(const uint32_t* kin, const uint32_t* vin, uint32_
     c.scratch = base;
     c.bucket_bytes = base + make_geometry(n, c.logb, kv).off_buckets;
     c.stream = stream;
-    cudaError_t e = dispatch_digit_prescan(desc->kind, c);
+    cudaError_t e = dispatch_digit_prescan(desc->kind, c, &c.rows_per);
     if (e == cudaSuccess) e = run_digit_postscan(c);
     if (e != cudaSuccess) return cuda_status(e);
   }
@@ -587,7 +589,7 @@ size_t wide_required_bytes(const Geometry& g, int key_bytes) { return key_bytes 
 // 32-bit path; everything else the 64-bit instances.
 gms_status multisplit_wide_impl(const void* kin, const void* vin, void* kout, void* vout, uint32_t n, int key_bytes,
                                 int value_bytes, const gms_bucket_desc64* desc, void* scratch, size_t scratch_bytes,
-                                cudaStream_t stream, uint32_t* starts = nullptr) {
+                                cudaStream_t stream, uint32_t* starts = nullptr, bool keep_matrix = false) {
   if (!valid_widths(key_bytes, value_bytes)) return GMS_ERROR_INVALID_VALUE;
   const bool kv = value_bytes != 0;
   if (key_bytes == 4 && value_bytes != 8) {
@@ -633,6 +635,7 @@ gms_status multisplit_wide_impl(const void* kin, const void* vin, void* kout, vo
   c.stream = stream;
   c.scratch_bytes = scratch_bytes;
   c.starts = starts;
+  c.keep_matrix = keep_matrix;
   if (key_bytes == 8) {
     c.bp64 = to_params64(desc);
     c.bucket_bytes = c.scratch + g.off_buckets;
@@ -738,6 +741,16 @@ cudaError_t run_scan(uint32_t* data, uint32_t m, uint64_t* status, ScratchHeader
   return launch_after_previous(scan_kernel, dim3(chunks), dim3(SCAN_THREADS), 0, stream, data, m, status, hdr);
 }
 
+cudaError_t run_scan_rows(uint32_t* rows, uint32_t num_buckets, uint32_t num_tiles, uint32_t per, uint64_t* status,
+                          ScratchHeader* hdr, cudaStream_t stream) {
+  const uint32_t ranges = (num_tiles + per - 1) / per;
+  const uint32_t blocks = num_buckets > SCAN_ROWS_COLS ? num_buckets / SCAN_ROWS_COLS : 1u;
+  return launch_after_previous(scan_rows_kernel, dim3(blocks), dim3(SCAN_ROWS_THREADS), 0, stream, rows, num_buckets,
+                               ranges, per, status, hdr);
+}
+
+uint32_t scan_rows_limit(uint32_t num_buckets) { return scan_rows_max_ranges(num_buckets); }
+
 void note_cuda_error(cudaError_t e) { g_last_cuda_error = int(e); }
 
 int device_sm_count() {
@@ -793,7 +806,7 @@ gms_status gms_multisplit_scratch_bytes(uint32_t max_elements, uint32_t num_buck
     return GMS_SUCCESS;
   }
   if (!valid_buckets(num_buckets, &logb)) return GMS_ERROR_UNSUPPORTED_BUCKETS;
-  *bytes = make_geometry(max_elements, logb, key_value != 0).bytes_full;
+  *bytes = make_geometry(max_elements, logb, key_value != 0).bytes_rows;
   return GMS_SUCCESS;
 }
 
@@ -994,7 +1007,8 @@ gms_status gms_multisplit_wide_scratch_bytes(uint32_t max_elements, uint32_t num
   if (bytes == nullptr || !valid_widths(key_bytes, value_bytes)) return GMS_ERROR_INVALID_VALUE;
   if (!valid_buckets(num_buckets, &logb)) return GMS_ERROR_UNSUPPORTED_BUCKETS;
   const bool kv = value_bytes != 0;
-  *bytes = make_geometry(max_elements, logb, kv, key_bytes / 4, kv ? value_bytes / 4 : 1).bytes_full;
+  const Geometry g = make_geometry(max_elements, logb, kv, key_bytes / 4, kv ? value_bytes / 4 : 1);
+  *bytes = key_bytes == 4 && value_bytes != 8 ? g.bytes_rows : g.bytes_full;
   return GMS_SUCCESS;
 }
 
@@ -1003,7 +1017,8 @@ gms_status gms_multisplit_wide(const void* d_key_in, const void* d_value_in, voi
                                void* d_scratch, size_t scratch_bytes, uint32_t* h_offsets, gms_stream_t stream) {
   uint32_t* starts = h_offsets != nullptr && n != 0 ? t_starts.get() : nullptr;
   gms_status st = multisplit_wide_impl(d_key_in, d_value_in, d_key_out, d_value_out, n, key_bytes, value_bytes, desc,
-                                       d_scratch, scratch_bytes, stream, starts);
+                                       d_scratch, scratch_bytes, stream, starts,
+                                       h_offsets != nullptr && starts == nullptr);
   if (st != GMS_SUCCESS || h_offsets == nullptr) return st;
   int logb = 0;
   valid_buckets(desc->num_buckets, &logb);

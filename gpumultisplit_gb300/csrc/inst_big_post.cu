@@ -4,6 +4,6 @@
 
 namespace gms {
 
-cudaError_t run_digit_postscan(const DigitPass& c) { GMS_DIGIT_SWITCH(digit_postscan_t, ) }
+cudaError_t run_digit_postscan(const DigitPass& c) { GMS_DIGIT_SWITCH((c), digit_postscan_t, ) }
 
 }  // namespace gms

@@ -50,6 +50,13 @@ inline uint32_t persistent_grid(Kernel k, int threads, uint32_t work, std::atomi
   return uint32_t(work < cap ? work : cap);
 }
 
+// A prescan's grid: no more blocks than ranges that one scan of the rows takes.
+inline uint32_t rows_grid(uint32_t grid, const uint32_t* rows, uint32_t num_buckets) {
+  if (rows == nullptr) return grid;
+  const uint32_t most = scan_rows_limit(num_buckets);
+  return grid < most ? grid : most;
+}
+
 // Stages of one multisplit with identifier policy P (descriptor kinds here;
 // user functors from the drop-in C++ headers).  `scratch` is laid out as
 // make_geometry(n, LOGB, KV).  bucket_bytes (n bytes, or null): for
@@ -218,7 +225,7 @@ template <class P, int LOGB, bool KV, int KW = 1, int VW = 1>
 cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<KW>* kout, ElemT<VW>* vout,
                               uint32_t n, const typename P::Params& params, unsigned char* scratch, int stages,
                               cudaStream_t stream, uint8_t* bucket_bytes = nullptr, size_t scratch_bytes = 0,
-                              uint32_t* starts = nullptr) {
+                              uint32_t* starts = nullptr, bool keep_matrix = true) {
   if constexpr (P::template CHEAP<KV>) bucket_bytes = nullptr;
   using S = TileShape<LOGB, KV, KW, VW>;
   using C = TileCfg<LOGB, S::WARPS, S::IPT, KV, KW, VW>;
@@ -234,19 +241,43 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
         launch_fused<C, P>(kin, vin, kout, vout, n, params, scratch, scratch_bytes, g, stream, starts, &launched);
     if (e != cudaSuccess || launched) return e;
   }
+  // Counts as rows: in the matrix's place, or beside it when the caller is to
+  // find the matrix and the scratch has the room.
+  uint32_t* rows = nullptr;
+  if (stages == STAGE_ALL && counts_as_rows(LOGB, g.num_tiles) && (!P::USES_SMEM || bucket_bytes != nullptr)) {
+    if (!keep_matrix) {
+      rows = matrix;
+    } else {
+      const size_t off = bucket_bytes != nullptr ? g.bytes_full : g.off_buckets;
+      if (scratch_bytes >= off + size_t(g.m) * 4) rows = reinterpret_cast<uint32_t*>(scratch + off);
+    }
+  }
+  uint32_t* const counts = rows != nullptr ? rows : matrix;
+  uint32_t* const matrix_out = rows != matrix && rows != nullptr ? matrix : nullptr;
+  // The postscan's blocks: one per tile, then those that fill in the matrix.
+  const uint32_t post_blocks =
+      g.num_tiles + (matrix_out != nullptr ? (g.num_tiles + MATRIX_TILES - 1) / MATRIX_TILES : 0u);
+  uint32_t rows_per = 0;  // tiles per range, known with the prescan's grid
+  auto choose_rows = [&](uint32_t grid) {
+    if (rows == nullptr) return;
+    rows_per = (g.num_tiles + grid - 1) / grid;
+  };
+
   if constexpr (KW == 2) {
     if (bucket_bytes == nullptr) return cudaErrorInvalidValue;
     if (stages & STAGE_PRESCAN) {
       static std::atomic<int> per_sm{0};
       auto kern = prescan64_kernel<C, P>;
-      const uint32_t grid = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm);
-      kern<<<grid, C::THREADS, 0, stream>>>(kin, n, g.num_tiles, matrix, params, hdr, status, g.num_chunks,
-                                            bucket_bytes);
+      const uint32_t grid = rows_grid(persistent_grid(kern, C::THREADS, g.num_tiles, per_sm), rows, C::B);
+      choose_rows(grid);
+      kern<<<grid, C::THREADS, 0, stream>>>(kin, n, g.num_tiles, counts, params, hdr, status, g.num_chunks,
+                                            bucket_bytes, rows_per);
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
     }
     if (stages & STAGE_SCAN) {
-      cudaError_t e = run_scan(matrix, g.m, status, hdr, stream);
+      cudaError_t e = rows_per != 0 ? run_scan_rows(rows, C::B, g.num_tiles, rows_per, status, hdr, stream)
+                                    : run_scan(matrix, g.m, status, hdr, stream);
       if (e != cudaSuccess) return e;
     }
     if (stages & STAGE_POSTSCAN) {
@@ -258,22 +289,24 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
       if (e != cudaSuccess) return e;
       const uint32_t wave = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem);
       const uint32_t dist = (GMS_PREFETCH_WAVES * wave) / 4u;
-      return launch_after_previous(kern, dim3(g.num_tiles), dim3(C::THREADS), smem, stream, kin, vin, kout, vout, n,
-                                   g.num_tiles, matrix, params, hdr, dist, bucket_bytes, starts);
+      return launch_after_previous(kern, dim3(post_blocks), dim3(C::THREADS), smem, stream, kin, vin, kout, vout, n,
+                                   g.num_tiles, counts, params, hdr, dist, bucket_bytes, starts, rows_per, matrix_out);
     }
     return cudaSuccess;
   } else {
   if (stages & STAGE_PRESCAN) {
     static std::atomic<int> per_sm{0};
     auto kern = prescan_kernel<C, P>;
-    const uint32_t grid = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm);
-    kern<<<grid, C::THREADS, 0, stream>>>(kin, n, g.num_tiles, matrix, params, hdr, status, g.num_chunks,
-                                          bucket_bytes);
+    const uint32_t grid = rows_grid(persistent_grid(kern, C::THREADS, g.num_tiles, per_sm), rows, C::B);
+    choose_rows(grid);
+    kern<<<grid, C::THREADS, 0, stream>>>(kin, n, g.num_tiles, counts, params, hdr, status, g.num_chunks,
+                                          bucket_bytes, rows_per);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   if (stages & STAGE_SCAN) {
-    cudaError_t e = run_scan(matrix, g.m, status, hdr, stream);
+    cudaError_t e = rows_per != 0 ? run_scan_rows(rows, C::B, g.num_tiles, rows_per, status, hdr, stream)
+                                  : run_scan(matrix, g.m, status, hdr, stream);
     if (e != cudaSuccess) return e;
   }
   if constexpr (!P::template CHEAP<KV>) {
@@ -287,8 +320,8 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
       if (e != cudaSuccess) return e;
       const uint32_t wave = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem);
       const uint32_t dist = (GMS_PREFETCH_WAVES * wave) / 4u;
-      return launch_after_previous(kern, dim3(g.num_tiles), dim3(C::THREADS), smem, stream, kin, vin, kout, vout, n,
-                                   g.num_tiles, matrix, params, hdr, dist, bucket_bytes, starts);
+      return launch_after_previous(kern, dim3(post_blocks), dim3(C::THREADS), smem, stream, kin, vin, kout, vout, n,
+                                   g.num_tiles, counts, params, hdr, dist, bucket_bytes, starts, rows_per, matrix_out);
     }
   }
   if ((stages & STAGE_POSTSCAN) && P::USES_SMEM) {
@@ -313,8 +346,9 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
     // Prefetch distance: a fraction of the number of blocks resident at once (one wave).
     const uint32_t wave = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm, smem);
     const uint32_t dist = (GMS_PREFETCH_WAVES * wave) / 4u;
-    e = launch_after_previous(kern, dim3(g.num_tiles), dim3(C::THREADS), smem, stream, kin, vin, kout, vout, n,
-                              g.num_tiles, matrix, params, hdr, dist, static_cast<const uint8_t*>(nullptr), starts);
+    e = launch_after_previous(kern, dim3(post_blocks), dim3(C::THREADS), smem, stream, kin, vin, kout, vout, n,
+                              g.num_tiles, counts, params, hdr, dist, static_cast<const uint8_t*>(nullptr), starts,
+                              rows_per, matrix_out);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -324,7 +358,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
 template <int KIND, int LOGB, bool KV>
 cudaError_t run_multisplit_t(const MsCall& c, int stages) {
   return launch_multisplit<DescPolicy<KIND, LOGB>, LOGB, KV>(c.kin, c.vin, c.kout, c.vout, c.n, c.bp, c.scratch,
-                                                             stages, c.stream, c.bucket_bytes, c.scratch_bytes, c.starts);
+                                                             stages, c.stream, c.bucket_bytes, c.scratch_bytes, c.starts, c.keep_matrix);
 }
 
 template <int KIND, bool KV>
@@ -359,10 +393,10 @@ cudaError_t run_multisplit_wide_t(const MsCallWide& c, int stages) {
   if constexpr (KW == 2)
     return launch_multisplit<DescPolicy64<KIND, LOGB>, LOGB, KV, KW, VW>(kin, vin, kout, vout, c.n, c.bp64,
                                                                            c.scratch, stages, c.stream,
-                                                                           c.bucket_bytes, c.scratch_bytes, c.starts);
+                                                                           c.bucket_bytes, c.scratch_bytes, c.starts, c.keep_matrix);
   else
     return launch_multisplit<DescPolicy<KIND, LOGB>, LOGB, KV, KW, VW>(kin, vin, kout, vout, c.n, c.bp, c.scratch,
-                                                                         stages, c.stream, c.bucket_bytes, c.scratch_bytes, c.starts);
+                                                                         stages, c.stream, c.bucket_bytes, c.scratch_bytes, c.starts, c.keep_matrix);
 }
 
 template <int KIND, int LOGB>
@@ -518,7 +552,7 @@ cudaError_t run_histogram(const uint32_t* keys, uint32_t n, int logb, const Buck
 
 // ------------------------------------------- more than 256 buckets
 template <int KIND, int LOGB, bool KV>
-cudaError_t digit_prescan_scan_t(const DigitPass& c) {
+cudaError_t digit_prescan_scan_t(const DigitPass& c, uint32_t* rows_per) {
   using S = TileShape<LOGB, KV>;
   using C = TileCfg<LOGB, S::WARPS, S::IPT, KV>;
   const Geometry g = make_geometry(c.n, LOGB, KV);
@@ -529,11 +563,14 @@ cudaError_t digit_prescan_scan_t(const DigitPass& c) {
   auto* matrix = reinterpret_cast<uint32_t*>(c.scratch + g.off_matrix);
   static std::atomic<int> per_sm{0};
   auto kern = prescan_kernel<C, DigitPolicy<KIND, LOGB>>;
-  const uint32_t grid = persistent_grid(kern, C::THREADS, g.num_tiles, per_sm);
+  uint32_t* const rows = counts_as_rows(LOGB, g.num_tiles) ? matrix : nullptr;  // nothing reads the matrix afterwards
+  const uint32_t grid = rows_grid(persistent_grid(kern, C::THREADS, g.num_tiles, per_sm), rows, C::B);
+  *rows_per = rows != nullptr ? (g.num_tiles + grid - 1) / grid : 0u;
   kern<<<grid, C::THREADS, 0, c.stream>>>(c.kin, c.n, g.num_tiles, matrix, c.bp, hdr, status, g.num_chunks,
-                                          c.bucket_bytes);
+                                          c.bucket_bytes, *rows_per);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
+  if (rows != nullptr) return run_scan_rows(rows, C::B, g.num_tiles, *rows_per, status, hdr, c.stream);
   return run_scan(matrix, g.m, status, hdr, c.stream);
 }
 
@@ -557,25 +594,25 @@ cudaError_t digit_postscan_t(const DigitPass& c) {
   const uint32_t dist = (GMS_PREFETCH_WAVES * wave) / 4u;
   return launch_after_previous(kern, dim3(g.num_tiles), dim3(C::THREADS), smem, c.stream, c.kin, c.vin, c.kout,
                                c.vout, c.n, g.num_tiles, matrix, c.bp, hdr, dist, c.bucket_bytes,
-                               static_cast<uint32_t*>(nullptr));
+                               static_cast<uint32_t*>(nullptr), c.rows_per, static_cast<uint32_t*>(nullptr));
 }
 
-#define GMS_DIGIT_SWITCH(FN, ...)                                 \
+#define GMS_DIGIT_SWITCH(ARGS, FN, ...)                           \
   switch (c.logb) {                                               \
-    case 1: return c.kv ? FN<__VA_ARGS__ 1, true>(c) : FN<__VA_ARGS__ 1, false>(c); \
-    case 2: return c.kv ? FN<__VA_ARGS__ 2, true>(c) : FN<__VA_ARGS__ 2, false>(c); \
-    case 3: return c.kv ? FN<__VA_ARGS__ 3, true>(c) : FN<__VA_ARGS__ 3, false>(c); \
-    case 4: return c.kv ? FN<__VA_ARGS__ 4, true>(c) : FN<__VA_ARGS__ 4, false>(c); \
-    case 5: return c.kv ? FN<__VA_ARGS__ 5, true>(c) : FN<__VA_ARGS__ 5, false>(c); \
-    case 6: return c.kv ? FN<__VA_ARGS__ 6, true>(c) : FN<__VA_ARGS__ 6, false>(c); \
-    case 7: return c.kv ? FN<__VA_ARGS__ 7, true>(c) : FN<__VA_ARGS__ 7, false>(c); \
-    case 8: return c.kv ? FN<__VA_ARGS__ 8, true>(c) : FN<__VA_ARGS__ 8, false>(c); \
+    case 1: return c.kv ? FN<__VA_ARGS__ 1, true> ARGS : FN<__VA_ARGS__ 1, false> ARGS; \
+    case 2: return c.kv ? FN<__VA_ARGS__ 2, true> ARGS : FN<__VA_ARGS__ 2, false> ARGS; \
+    case 3: return c.kv ? FN<__VA_ARGS__ 3, true> ARGS : FN<__VA_ARGS__ 3, false> ARGS; \
+    case 4: return c.kv ? FN<__VA_ARGS__ 4, true> ARGS : FN<__VA_ARGS__ 4, false> ARGS; \
+    case 5: return c.kv ? FN<__VA_ARGS__ 5, true> ARGS : FN<__VA_ARGS__ 5, false> ARGS; \
+    case 6: return c.kv ? FN<__VA_ARGS__ 6, true> ARGS : FN<__VA_ARGS__ 6, false> ARGS; \
+    case 7: return c.kv ? FN<__VA_ARGS__ 7, true> ARGS : FN<__VA_ARGS__ 7, false> ARGS; \
+    case 8: return c.kv ? FN<__VA_ARGS__ 8, true> ARGS : FN<__VA_ARGS__ 8, false> ARGS; \
     default: return cudaErrorInvalidValue;                        \
   }
 
 template <int KIND>
-cudaError_t run_digit_prescan_scan(const DigitPass& c) {
-  GMS_DIGIT_SWITCH(digit_prescan_scan_t, KIND,)
+cudaError_t run_digit_prescan_scan(const DigitPass& c, uint32_t* rows_per) {
+  GMS_DIGIT_SWITCH((c, rows_per), digit_prescan_scan_t, KIND,)
 }
 
 template <int KIND>
@@ -623,7 +660,7 @@ cudaError_t run_big_offsets(const uint32_t* sorted_keys, uint32_t n, const Bucke
                                              int32_t*, cudaStream_t);
 
 #define GMS_INSTANTIATE_BIG(K)                                                           \
-  template cudaError_t gms::run_digit_prescan_scan<K>(const gms::DigitPass&);           \
+  template cudaError_t gms::run_digit_prescan_scan<K>(const gms::DigitPass&, uint32_t*);           \
   template cudaError_t gms::run_big_histogram<K>(const uint32_t*, uint32_t, const gms::BucketParams&, uint32_t*, \
                                                  cudaStream_t);                                                 \
   template cudaError_t gms::run_big_offsets<K>(const uint32_t*, uint32_t, const gms::BucketParams&, uint32_t*, \

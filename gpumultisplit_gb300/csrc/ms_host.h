@@ -82,6 +82,13 @@ constexpr uint32_t kScanChunk = 256u * GMS_SCAN_IPT;  // SCAN_CHUNK in scan_kern
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// Whether a one-call multisplit keeps its counts as rows (prescan_kernel): from
+// 65 buckets up, where reading the matrix costs the postscan most (us, matrix /
+// rows: 2^25 keys 64 buckets 102 / 102, 128 116 / 109, 256 148 / 123; pairs 32
+// buckets 116 / 121, 64 125 / 127, 128 138 / 137, 256 183 / 165), and from 512
+// tiles up; fewer run as one launch where they can, and over the matrix where not.
+constexpr bool counts_as_rows(int logb, uint32_t num_tiles) { return logb >= 7 && num_tiles >= 512; }
+
 // Scratch layout of one multisplit: [header 256 B][count matrix u32 x B*tiles][scan status u64 x chunks].
 // The matrix always starts at byte 256, whatever n is.
 struct Geometry {
@@ -93,7 +100,8 @@ struct Geometry {
   size_t off_matrix = 0;
   size_t bytes = 0;         // what every identifier needs
   size_t off_buckets = 0;   // one byte per key, used by costly identifiers when the scratch has room
-  size_t bytes_full = 0;    // bytes plus the bucket bytes (what gms_multisplit_scratch_bytes reports)
+  size_t bytes_full = 0;    // bytes plus the bucket bytes
+  size_t bytes_rows = 0;    // plus the counts as rows beside the matrix (what gms_multisplit_scratch_bytes reports)
 };
 
 // kw / vw: 32-bit words per key / value (2 for 64-bit elements).
@@ -108,6 +116,7 @@ inline Geometry make_geometry(uint32_t n, int logb, bool kv, int kw = 1, int vw 
   g.bytes = align_up(g.off_status + size_t(g.num_chunks) * 8, 256);
   g.off_buckets = g.bytes;
   g.bytes_full = align_up(g.off_buckets + size_t(n), 256);
+  g.bytes_rows = align_up(g.bytes_full + (counts_as_rows(logb, g.num_tiles) ? size_t(g.m) * 4 : 0), 256);
   return g;
 }
 
@@ -141,6 +150,7 @@ struct MsCall {
   uint8_t* bucket_bytes = nullptr;   // in scratch, or null (see launch_multisplit)
   size_t scratch_bytes = 0;          // bytes at scratch
   uint32_t* starts = nullptr;        // pinned host memory for 2^logb bucket starts, or null
+  bool keep_matrix = true;           // the count matrix holds the global offsets afterwards
 };
 
 // Runs the requested stages (a mask of Stage) of one multisplit.  Defined per
@@ -168,6 +178,7 @@ struct MsCallWide {
   uint8_t* bucket_bytes = nullptr;
   size_t scratch_bytes = 0;          // bytes at scratch
   uint32_t* starts = nullptr;        // pinned host memory for 2^logb bucket starts, or null
+  bool keep_matrix = true;           // the count matrix holds the global offsets afterwards
 };
 
 // Defined per identifier kind in inst_wide.cu (compiled once per kind).
@@ -192,13 +203,15 @@ struct DigitPass {
   BucketParamsBig bp{};
   unsigned char* scratch = nullptr;
   uint8_t* bucket_bytes = nullptr;
+  uint32_t rows_per = 0;  // tiles per range of the counts' rows; 0: the bucket-major matrix
   cudaStream_t stream = nullptr;
 };
 
 // Prescan (identifier evaluated, digit kept as a byte) and scan of a digit
 // pass; defined per kind in inst_big.cu.
+// *rows_per: the postscan's (DigitPass::rows_per).
 template <int KIND>
-cudaError_t run_digit_prescan_scan(const DigitPass& c);
+cudaError_t run_digit_prescan_scan(const DigitPass& c, uint32_t* rows_per);
 // Postscan of a digit pass from the bytes (inst_big_post.cu).
 cudaError_t run_digit_postscan(const DigitPass& c);
 // Adds the count of every whole bucket id in [0, p.num_buckets) into hist
@@ -236,6 +249,12 @@ cudaError_t launch_after_previous(void (*kern)(KArgs...), dim3 grid, dim3 block,
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
+
+// Scans the range totals in a prescan's rows (scan_kernels.cuh); at most
+// scan_rows_limit(num_buckets) ranges.
+cudaError_t run_scan_rows(uint32_t* rows, uint32_t num_buckets, uint32_t num_tiles, uint32_t per, uint64_t* status,
+                          ScratchHeader* hdr, cudaStream_t stream);
+uint32_t scan_rows_limit(uint32_t num_buckets);
 
 cudaError_t run_scan(uint32_t* data, uint32_t m, uint64_t* status, ScratchHeader* hdr, cudaStream_t stream);
 

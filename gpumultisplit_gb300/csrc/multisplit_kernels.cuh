@@ -232,18 +232,69 @@ __device__ __forceinline__ void count_tiles(const uint32_t* __restrict__ keys, u
 // bucket is also stored there as one byte, so the postscan need not evaluate
 // the identifier again.
 //
-// Each block counts a contiguous run of tiles and keeps the counts of
+// Each block counts a contiguous run of tiles, as even as whole tiles allow, and keeps the counts of
 // PRESCAN_GROUP consecutive tiles in shared memory, then writes them bucket by
 // bucket: a warp stores whole runs of consecutive matrix words (the matrix is
 // bucket-major) instead of one scattered word per bucket and tile.
+//
+// rows_per != 0 (the one-call path): the counts go into rows instead,
+// counts[tile * B + b], one coalesced store per tile.  A block's range is then
+// rows_per tiles, each row holds the counts of the range's earlier tiles, and
+// the range's first row, whose sums would be zero, the range's totals; only
+// those rows are scanned (scan_rows_kernel), and the postscan adds the two rows
+// of its tile, each read as whole sectors.  The bucket-major matrix made the
+// postscan read a sector for every bucket: of its 145 us for 2^25 pairs at 256
+// buckets (113 for keys) 18 (16) went into those loads, and the scan ran over
+// all counts.
 constexpr uint32_t PRESCAN_GROUP = 8;
+
+template <class C>
+struct PrescanCounts {
+  static constexpr uint32_t B = C::B;
+  static constexpr uint32_t G = PRESCAN_GROUP;
+  uint32_t* counts;
+  uint32_t* s_cnt;  // B * G words
+  uint32_t num_tiles, first, last;
+  bool rows;
+  uint32_t run;     // rows: count of bucket tid in the range so far
+
+  __device__ __forceinline__ PrescanCounts(uint32_t* counts_, uint32_t* s_cnt_, uint32_t num_tiles_, uint32_t rows_per)
+      : counts(counts_), s_cnt(s_cnt_), num_tiles(num_tiles_), rows(rows_per != 0), run(0) {
+    const uint32_t per = rows ? rows_per : (num_tiles + gridDim.x - 1) / gridDim.x;
+    first = min(blockIdx.x * per, num_tiles);
+    last = min(first + per, num_tiles);
+  }
+  // Called by all threads after each tile; thread tid < B has the tile's count of bucket tid.
+  __device__ __forceinline__ void done(uint32_t tile, uint32_t total) {
+    const uint32_t tid = threadIdx.x;
+    if (rows) {
+      if (tid < B) {
+        if (tile != first) counts[tile * B + tid] = run;
+        run += total;
+        if (tile + 1 == last) counts[first * B + tid] = run;
+      }
+      return;
+    }
+    const uint32_t g = (tile - first) % G;
+    if (tid < B) s_cnt[tid * G + g] = total;
+    if (g == G - 1 || tile + 1 == last) {
+      const uint32_t group_first = tile - g;
+      __syncthreads();
+      for (uint32_t i = tid; i < B * G; i += C::THREADS) {
+        const uint32_t t = group_first + i % G;
+        if (t < last) counts[(i / G) * num_tiles + t] = s_cnt[i];
+      }
+      __syncthreads();
+    }
+  }
+};
 
 template <class C, class P>
 __global__ void __launch_bounds__(C::THREADS) prescan_kernel(const uint32_t* __restrict__ keys, uint32_t n,
                                                              uint32_t num_tiles, uint32_t* __restrict__ counts,
                                                              typename P::Params bp, ScratchHeader* hdr,
                                                              uint64_t* __restrict__ status, uint32_t num_chunks,
-                                                             uint8_t* __restrict__ bucket_bytes) {
+                                                             uint8_t* __restrict__ bucket_bytes, uint32_t rows_per) {
   griddep_launch_dependents();  // the scan may be scheduled now; it waits for this grid
   using Counter = KeyCounter<C::LOGB, typename P::Id>;
   constexpr uint32_t G = PRESCAN_GROUP;
@@ -266,31 +317,15 @@ __global__ void __launch_bounds__(C::THREADS) prescan_kernel(const uint32_t* __r
   Counter counter(P::make(bp, s_split), s_hist);
   counter.clear_shared();
   __syncthreads();
-  // This block's tiles: [first, last), a whole number of groups.
-  const uint32_t per = ((num_tiles + gridDim.x - 1) / gridDim.x + G - 1) / G * G;
-  const uint32_t first = min(blockIdx.x * per, num_tiles);
-  const uint32_t last = min(first + per, num_tiles);
-  auto flush = [&](uint32_t group_first) {
-    __syncthreads();
-    for (uint32_t i = tid; i < C::B * G; i += C::THREADS) {
-      const uint32_t t = group_first + i % G;
-      if (t < last) counts[(i / G) * num_tiles + t] = s_cnt[i];
-    }
-    __syncthreads();
-  };
-  auto done = [&](uint32_t tile) {
-    const uint32_t total = counter.block_total();
-    const uint32_t g = (tile - first) % G;
-    if (tid < C::B) s_cnt[tid * G + g] = total;
-    if (g == G - 1 || tile + 1 == last) flush(tile - g);
-  };
+  PrescanCounts<C> out(counts, s_cnt, num_tiles, rows_per);
+  auto done = [&](uint32_t tile) { out.done(tile, counter.block_total()); };
   if constexpr (!P::template CHEAP<C::KV>) {
     if (bucket_bytes != nullptr) {
-      count_tiles<C::THREADS, C::IPT, true>(keys, n, first, 1u, counter, done, bucket_bytes, last);
+      count_tiles<C::THREADS, C::IPT, true>(keys, n, out.first, 1u, counter, done, bucket_bytes, out.last);
       return;
     }
   }
-  count_tiles<C::THREADS, C::IPT>(keys, n, first, 1u, counter, done, nullptr, last);
+  count_tiles<C::THREADS, C::IPT>(keys, n, out.first, 1u, counter, done, nullptr, out.last);
 }
 
 // ------------------------------------------------ prescan, 64-bit keys
@@ -313,7 +348,7 @@ __global__ void __launch_bounds__(C::THREADS) prescan64_kernel(const uint64_t* _
                                                                uint32_t num_tiles, uint32_t* __restrict__ counts,
                                                                typename P::Params bp, ScratchHeader* hdr,
                                                                uint64_t* __restrict__ status, uint32_t num_chunks,
-                                                               uint8_t* __restrict__ bucket_bytes) {
+                                                               uint8_t* __restrict__ bucket_bytes, uint32_t rows_per) {
   griddep_launch_dependents();  // the scan may be scheduled now; it waits for this grid
   using Counter = KeyCounter<C::LOGB, typename P::Id>;
   constexpr uint32_t G = PRESCAN_GROUP;
@@ -336,18 +371,8 @@ __global__ void __launch_bounds__(C::THREADS) prescan64_kernel(const uint64_t* _
   Counter counter(P::make(bp, s_split), s_hist);
   counter.clear_shared();
   __syncthreads();
-  const uint32_t per = ((num_tiles + gridDim.x - 1) / gridDim.x + G - 1) / G * G;
-  const uint32_t first = min(blockIdx.x * per, num_tiles);
-  const uint32_t last = min(first + per, num_tiles);
-  auto flush = [&](uint32_t group_first) {
-    __syncthreads();
-    for (uint32_t i = tid; i < C::B * G; i += C::THREADS) {
-      const uint32_t t = group_first + i % G;
-      if (t < last) counts[(i / G) * num_tiles + t] = s_cnt[i];
-    }
-    __syncthreads();
-  };
-
+  PrescanCounts<C> out(counts, s_cnt, num_tiles, rows_per);
+  const uint32_t first = out.first, last = out.last;
   const bool vec_ok = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
   const uint32_t full_tiles = vec_ok ? min(n / TILE, last) : 0u;
   uint4 cur[NV];
@@ -357,14 +382,14 @@ __global__ void __launch_bounds__(C::THREADS) prescan64_kernel(const uint64_t* _
     if (tile + 1 < full_tiles) load_tile64<C::THREADS, C::IPT>(keys, (tile + 1) * TILE, nxt);
     const uint32_t base = tile * TILE;
     if (tile < full_tiles) {
-      uint16_t* out = reinterpret_cast<uint16_t*>(bucket_bytes + base);
+      uint16_t* bytes = reinterpret_cast<uint16_t*>(bucket_bytes + base);
 #pragma unroll
       for (int k = 0; k < NV; ++k) {
         const uint32_t b0 = counter.ident(uint64_t(cur[k].x) | (uint64_t(cur[k].y) << 32));
         const uint32_t b1 = counter.ident(uint64_t(cur[k].z) | (uint64_t(cur[k].w) << 32));
         counter.template add_bucket<0>(b0, true);
         counter.template add_bucket<1>(b1, true);
-        out[uint32_t(k) * C::THREADS + tid] = uint16_t(b0 | (b1 << 8));
+        bytes[uint32_t(k) * C::THREADS + tid] = uint16_t(b0 | (b1 << 8));
       }
     } else {
       const uint32_t cnt = min(TILE, n - base);
@@ -377,10 +402,7 @@ __global__ void __launch_bounds__(C::THREADS) prescan64_kernel(const uint64_t* _
         if (valid) bucket_bytes[base + i] = uint8_t(b);
       }
     }
-    const uint32_t total = counter.block_total();
-    const uint32_t g = (tile - first) % G;
-    if (tid < C::B) s_cnt[tid * G + g] = total;
-    if (g == G - 1 || tile + 1 == last) flush(tile - g);
+    out.done(tile, counter.block_total());
 #pragma unroll
     for (int k = 0; k < NV; ++k) cur[k] = nxt[k];
   }
@@ -511,6 +533,45 @@ struct MatrixOffsets {
     return GivenOffset{tid < num_buckets ? job.offsets[tid * job.num_tiles + job.tile] - job.bias : 0u};
   }
 };
+
+// The same from the prescan's rows (per tiles a range, see prescan_kernel);
+// per == 0: job.offsets is the bucket-major matrix.
+struct RowOffsets {
+  uint32_t per;
+
+  template <class Job>
+  __device__ __forceinline__ GivenOffset operator()(const Job& job, uint32_t tid, uint32_t num_buckets) const {
+    if (per == 0) return MatrixOffsets()(job, tid, num_buckets);
+    if (tid >= num_buckets) return GivenOffset{0u};
+    const uint32_t first = job.tile - job.tile % per;
+    const uint32_t range = job.offsets[first * num_buckets + tid];
+    return GivenOffset{job.tile == first ? range : range + job.offsets[job.tile * num_buckets + tid]};
+  }
+};
+
+// Tiles whose offsets one block moves from the rows to the matrix.
+constexpr uint32_t MATRIX_TILES = 32;
+
+// Fills the bucket-major matrix that the caller sees from the rows, for tiles
+// [t0, t0 + MATRIX_TILES): through shared memory, whole rows in and runs of 32
+// words out.  Extra blocks of the postscan's grid do this while its last tiles
+// drain; done by every eighth tile's own block it took 85 us of a 1360 us call
+// (2^28 pairs, 256 buckets).
+template <uint32_t B>
+__device__ __forceinline__ void rows_to_matrix(const uint32_t* __restrict__ rows, uint32_t* __restrict__ matrix,
+                                               uint32_t num_tiles, uint32_t per, uint32_t t0, uint32_t* s) {
+  const uint32_t tiles = min(MATRIX_TILES, num_tiles - t0);
+  for (uint32_t i = threadIdx.x; i < tiles * B; i += blockDim.x) {
+    const uint32_t t = t0 + i / B, b = i % B;
+    const uint32_t first = t - t % per;
+    s[(i / B) * (B + 1) + b] = rows[first * B + b] + (t != first ? rows[t * B + b] : 0u);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < MATRIX_TILES * B; i += blockDim.x) {
+    const uint32_t k = i % MATRIX_TILES, b = i / MATRIX_TILES;
+    if (k < tiles) matrix[b * num_tiles + t0 + k] = s[k * (B + 1) + b];
+  }
+}
 
 // Phases 1-4 of the postscan for one staged tile.  FULL: the tile holds
 // exactly TILE keys, so no per-key validity test is needed.
@@ -774,10 +835,15 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
     }
   };
   if constexpr (C::ATOMIC) {
-    // Each warp walks its own stretch of the sorted order and checks, beside
-    // the stores, that (bucket, source) ascends from each position to the next.
-    // If it does not somewhere in the tile, every run is put in order and the
-    // tile is stored again.
+    // Each warp stores runs of RUN times 32 positions and checks beside it that
+    // (bucket, source) ascends from each position to the next, by a shuffle;
+    // from run to run one thread each checks.  If it does not somewhere in the
+    // tile, every bucket's run is put in order and the tile is stored again.
+    // Longer runs leave fewer places between them to check (the 7-bit sort of
+    // 2^25 keys: 551 us at one, 543 at four); at 256 buckets, whose runs are
+    // shortest, pairs want the block's stores close together (the 8-bit sort of
+    // 2^25 pairs: 606 us at one, 638 at four).
+    constexpr uint32_t RUN = C::KV && LOGB == 8 ? 1 : 4;
     using IndexT = std::conditional_t<L::WORDS, uint32_t, uint16_t>;
     IndexT* s_idx = reinterpret_cast<IndexT*>(s_r);
     // (bucket << 16) | source of sorted position p.
@@ -792,11 +858,10 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
     };
     for (int attempt = 0; attempt < 2; ++attempt) {
       bool late = false;
-      uint32_t before = 0;  // entry of the position before this warp's slot, in lane 0
-      if (lane == 0 && wbase != 0 && (FULL || wbase < cnt)) before = entry(wbase - 1);
+      uint32_t before = 0;  // lane 0: entry of the position before its slot
 #pragma unroll
       for (int j = 0; j < IPT; ++j) {
-        const uint32_t p = wbase + uint32_t(j) * 32u + lane;
+        const uint32_t p = (uint32_t(j) / RUN * C::WARPS + warp) * (32u * RUN) + uint32_t(j) % RUN * 32u + lane;
         uint32_t at = ~0u;
         if (FULL || p < cnt) {
           at = entry(p);
@@ -804,9 +869,10 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
           store(p, src, s_k[src], at >> 16);
         }
         const uint32_t left = __shfl_sync(~0u, at, (lane + 31u) & 31u);
-        late |= (lane == 0 ? before : left) > at;
-        before = left;  // lane 0: the slot's last
+        late |= (lane != 0 ? left : j % RUN == 0 ? 0u : before) > at;
+        before = left;
       }
+      for (uint32_t p = 32u * RUN * (tid + 1u); p < cnt; p += 32u * RUN * C::THREADS) late |= entry(p - 1) > entry(p);
       if (!__syncthreads_or(late)) break;
       if (tid < B) {  // s_wh[b] of warp 0 is the start of bucket b's run
         const uint32_t first = s_wh[tid], last = tid + 1 < B ? uint32_t(s_wh[tid + 1]) : cnt;
@@ -1003,11 +1069,11 @@ __device__ __forceinline__ void postscan_run(uint32_t first, uint32_t last, uint
   }
 }
 
-// The bucket starts (column 0 of the scanned matrix), stored by the block of
-// tile 0 where the caller wants them: pinned host memory (capi.cu).
-__device__ __forceinline__ void store_starts(uint32_t* starts, const uint32_t* offsets, uint32_t num_tiles,
+// The bucket starts (column 0 of the scanned matrix, row 0 of the rows), stored
+// by the block of tile 0 where the caller wants them: pinned host memory (capi.cu).
+__device__ __forceinline__ void store_starts(uint32_t* starts, const uint32_t* offsets, uint32_t stride,
                                              uint32_t num_buckets) {
-  if (starts != nullptr && threadIdx.x < num_buckets) starts[threadIdx.x] = offsets[threadIdx.x * num_tiles];
+  if (starts != nullptr && threadIdx.x < num_buckets) starts[threadIdx.x] = offsets[threadIdx.x * stride];
 }
 
 // Plain postscan: one block per tile of one multisplit.  GIVEN: the buckets
@@ -1017,15 +1083,21 @@ __global__ void __launch_bounds__(C::THREADS, (PostLayout<C, P, GIVEN>::MIN_BLOC
     const typename C::KT* __restrict__ kin, const typename C::VT* __restrict__ vin, typename C::KT* __restrict__ kout,
     typename C::VT* __restrict__ vout, uint32_t n, uint32_t num_tiles, const uint32_t* __restrict__ offsets,
     typename P::Params bp, ScratchHeader* hdr, uint32_t prefetch_dist, const uint8_t* __restrict__ bucket_bytes,
-    uint32_t* starts) {
+    uint32_t* starts, uint32_t rows_per, uint32_t* matrix) {
   extern __shared__ __align__(128) unsigned char smem[];
   griddep_wait();  // launched while the scan finishes: its offsets are complete past this point
-  if (blockIdx.x == 0) store_starts(starts, offsets, num_tiles, C::B);
+  if (blockIdx.x >= num_tiles) {  // block-uniform
+    static_assert(PostLayout<C, P, GIVEN>::BYTES >= MATRIX_TILES * (C::B + 1) * 4, "the tile's area holds the rows");
+    rows_to_matrix<C::B>(offsets, matrix, num_tiles, rows_per, (blockIdx.x - num_tiles) * MATRIX_TILES,
+                         reinterpret_cast<uint32_t*>(smem));
+    return;
+  }
+  if (blockIdx.x == 0) store_starts(starts, offsets, rows_per != 0 ? 1u : num_tiles, C::B);
   const TileJob<typename P::Params, typename C::KT, typename C::VT> job{kin,        vin,     kout, vout,
                                         n,          num_tiles, blockIdx.x, offsets,
                                         0u,         prefetch_dist != 0 ? blockIdx.x + prefetch_dist : ~0u,
                                         bp,         0u,      bucket_bytes};
-  postscan_job<C, P, true, GIVEN>(job, hdr, smem);
+  postscan_job<C, P, true, GIVEN, RowOffsets>(job, hdr, smem, nullptr, RowOffsets{rows_per});
 }
 
 // Persistent plain postscan (identifiers with a shared area): block b runs
