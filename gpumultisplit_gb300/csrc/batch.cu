@@ -110,11 +110,13 @@ cudaError_t run_batch_warp_kind(int kind, const BatchClassLaunch& c) {
   }
 }
 
+// For the classes of a stage (eight measured no faster: 267 us for 512 segments
+// of 16 to 1 Mi pairs with four, 283 with eight); one more for the one-warp classes.
 constexpr int kSideStreams = 4;
 
 cudaError_t ensure_side_streams(gms_batch_s* b) {
   if (!b->side.empty()) return cudaSuccess;
-  for (int i = 0; i < kSideStreams; ++i) {
+  for (int i = 0; i < kSideStreams + 1; ++i) {
     cudaStream_t st = nullptr;
     cudaEvent_t ev = nullptr;
     cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
@@ -132,21 +134,24 @@ cudaError_t ensure_side_streams(gms_batch_s* b) {
   return e;
 }
 
-// Launches one stage of every class.  With side streams the classes (largest
-// first) are dealt round-robin to the side streams, which fork from and join
-// back into `s`, so a stage's kernels of different classes can run at once.
+// Launches one stage of every tiled class.  With side streams the classes
+// (largest first) are dealt round-robin to the side streams, which fork from
+// and join back into `s`, so a stage's kernels of different classes can run at
+// once.  between(): launched on `s` while the side streams run.
+template <class Between>
 cudaError_t launch_classes(gms_batch_s* b, BatchClassLaunch L, unsigned char* scratch, cudaStream_t s, int stage,
-                           bool fork) {
-  const size_t nc = b->classes.size();
-  const int lanes = fork && nc > 1 ? int(std::min<size_t>(nc, b->side.size())) : 0;
+                           bool fork, Between between) {
+  std::vector<size_t> order;
+  for (size_t i = 0; i < b->classes.size(); ++i)
+    if (!b->classes[i].warp) order.push_back(i);
+  const size_t nc = order.size();
+  const int lanes = fork && nc > 1 ? int(std::min<size_t>(nc, kSideStreams)) : 0;
   cudaError_t e = cudaSuccess;
   if (lanes > 0) {
     e = cudaEventRecord(b->events.back(), s);
     for (int i = 0; e == cudaSuccess && i < lanes; ++i) e = cudaStreamWaitEvent(b->side[i], b->events.back(), 0);
     if (e != cudaSuccess) return e;
   }
-  std::vector<size_t> order(nc);
-  for (size_t i = 0; i < nc; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(),
                    [&](size_t x, size_t y) { return b->classes[x].work() > b->classes[y].work(); });
   for (size_t k = 0; k < nc; ++k) {
@@ -155,18 +160,12 @@ cudaError_t launch_classes(gms_batch_s* b, BatchClassLaunch L, unsigned char* sc
     L.kv = c.kv;
     L.variant = c.variant;
     L.stream = lanes > 0 ? b->side[k % size_t(lanes)] : s;
-    if (c.warp) {  // one kernel does the whole multisplit: launched with the postscans
-      if (stage != STAGE_POSTSCAN) continue;
-      L.seg_ids = reinterpret_cast<const uint32_t*>(scratch + c.map_off);
-      L.class_tiles = uint32_t(c.seg_ids.size());
-      e = run_batch_warp_kind(c.kind, L);
-    } else {
-      L.tile_map = reinterpret_cast<const uint2*>(scratch + c.map_off);
-      L.class_tiles = uint32_t(c.tiles.size());
-      e = run_batch_class(c.kind, L, stage);
-    }
+    L.tile_map = reinterpret_cast<const uint2*>(scratch + c.map_off);
+    L.class_tiles = uint32_t(c.tiles.size());
+    e = run_batch_class(c.kind, L, stage);
     if (e != cudaSuccess) return e;
   }
+  e = between();
   for (int i = 0; e == cudaSuccess && i < lanes; ++i) {
     e = cudaEventRecord(b->events[i], b->side[i]);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b->events[i], 0);
@@ -174,34 +173,69 @@ cudaError_t launch_classes(gms_batch_s* b, BatchClassLaunch L, unsigned char* sc
   return e;
 }
 
-// The launch sequence of one run: reset the error word, prescan every class,
-// scan every group (ticket and status words reset first), postscan every class.
+// Launches the one-warp classes, whose single kernel does the whole multisplit.
+cudaError_t launch_warp_classes(gms_batch_s* b, BatchClassLaunch L, unsigned char* scratch, cudaStream_t s) {
+  L.stream = s;
+  for (const BatchClass& c : b->classes) {
+    if (!c.warp) continue;
+    L.logb = c.logb;
+    L.kv = c.kv;
+    L.variant = c.variant;
+    L.seg_ids = reinterpret_cast<const uint32_t*>(scratch + c.map_off);
+    L.class_tiles = uint32_t(c.seg_ids.size());
+    const cudaError_t e = run_batch_warp_kind(c.kind, L);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+// The launch sequence of one run: prescan every class, with the error word,
+// ticket and status words reset beside it, scan every group, postscan every
+// class.  With side streams the one-warp classes run on a stream of their own
+// beside all of it: eight such kernels of 5-15 us each used to end the run.
 cudaError_t launch_all(gms_batch_s* b, unsigned char* scratch, cudaStream_t s, bool fork = false) {
   auto* hdr = reinterpret_cast<ScratchHeader*>(scratch);
   auto* matrix = reinterpret_cast<uint32_t*>(scratch + b->off_matrix);
   auto* status = reinterpret_cast<uint64_t*>(scratch + b->off_status);
-  cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(ScratchHeader), s);
-  if (e != cudaSuccess) return e;
   BatchClassLaunch L;
   L.segs = reinterpret_cast<const SegDesc*>(scratch + b->off_segs);
   L.matrix = matrix;
   L.byte_area = scratch + b->off_bytes;
   L.hdr = hdr;
   L.stream = s;
-  for (int stage : {int(STAGE_PRESCAN), int(STAGE_POSTSCAN)}) {
-    if (stage == STAGE_POSTSCAN) {
-      for (const ScanGroup& g : b->groups) {
-        e = cudaMemsetAsync(&hdr->ticket, 0, sizeof(uint32_t), s);
-        if (e == cudaSuccess)
-          e = cudaMemsetAsync(status, 0, size_t((g.m + kScanChunk - 1) / kScanChunk) * sizeof(uint64_t), s);
-        if (e == cudaSuccess) e = run_scan(matrix + g.matrix_first, g.m, status, hdr, s);
-        if (e != cudaSuccess) return e;
-      }
-    }
-    e = launch_classes(b, L, scratch, s, stage, fork);
+  bool any_warp = false;
+  for (const BatchClass& c : b->classes) any_warp |= c.warp;
+  cudaStream_t warp_stream = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (any_warp && fork) {
+    warp_stream = b->side[kSideStreams];
+    e = cudaEventRecord(b->events.back(), s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(warp_stream, b->events.back(), 0);
+    if (e == cudaSuccess) e = launch_warp_classes(b, L, scratch, warp_stream);
+    if (e == cudaSuccess) e = cudaEventRecord(b->events[kSideStreams], warp_stream);
     if (e != cudaSuccess) return e;
   }
-  return cudaSuccess;
+  auto chunks = [](const ScanGroup& g) { return size_t((g.m + kScanChunk - 1) / kScanChunk); };
+  e = launch_classes(b, L, scratch, s, STAGE_PRESCAN, fork, [&] {
+    cudaError_t r = cudaMemsetAsync(scratch, 0, sizeof(ScratchHeader), s);
+    if (r == cudaSuccess && !b->groups.empty())
+      r = cudaMemsetAsync(status, 0, chunks(b->groups[0]) * sizeof(uint64_t), s);
+    return r;
+  });
+  if (e != cudaSuccess) return e;
+  for (size_t i = 0; i < b->groups.size(); ++i) {
+    const ScanGroup& g = b->groups[i];
+    if (i > 0) {
+      e = cudaMemsetAsync(&hdr->ticket, 0, sizeof(uint32_t), s);
+      if (e == cudaSuccess) e = cudaMemsetAsync(status, 0, chunks(g) * sizeof(uint64_t), s);
+    }
+    if (e == cudaSuccess) e = run_scan(matrix + g.matrix_first, g.m, status, hdr, s);
+    if (e != cudaSuccess) return e;
+  }
+  e = launch_classes(b, L, scratch, s, STAGE_POSTSCAN, fork, [] { return cudaSuccess; });
+  if (e != cudaSuccess) return e;
+  if (warp_stream != nullptr) return cudaStreamWaitEvent(s, b->events[kSideStreams], 0);
+  return any_warp ? launch_warp_classes(b, L, scratch, s) : cudaSuccess;
 }
 
 // Order of the queue's work list.  Counting (PRE) tiles run this many tiles

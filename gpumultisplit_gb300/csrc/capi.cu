@@ -430,14 +430,14 @@ gms_status check_big_desc(const gms_bucket_desc* d) {
   }
 }
 
-cudaError_t dispatch_digit_prescan(int kind, const DigitPass& c, uint32_t* rows_per) {
+cudaError_t dispatch_digit_prescan(int kind, const DigitPass& c, uint32_t* rows_per, bool* done) {
   switch (kind) {
-    case KIND_DELTA: return run_digit_prescan_scan<KIND_DELTA>(c, rows_per);
-    case KIND_DIV: return run_digit_prescan_scan<KIND_DIV>(c, rows_per);
-    case KIND_BITS: return run_digit_prescan_scan<KIND_BITS>(c, rows_per);
-    case KIND_RANGE: return run_digit_prescan_scan<KIND_RANGE>(c, rows_per);
-    case KIND_MASK: return run_digit_prescan_scan<KIND_MASK>(c, rows_per);
-    case KIND_EVEN_FLOAT: return run_digit_prescan_scan<KIND_EVEN_FLOAT>(c, rows_per);
+    case KIND_DELTA: return run_digit_prescan_scan<KIND_DELTA>(c, rows_per, done);
+    case KIND_DIV: return run_digit_prescan_scan<KIND_DIV>(c, rows_per, done);
+    case KIND_BITS: return run_digit_prescan_scan<KIND_BITS>(c, rows_per, done);
+    case KIND_RANGE: return run_digit_prescan_scan<KIND_RANGE>(c, rows_per, done);
+    case KIND_MASK: return run_digit_prescan_scan<KIND_MASK>(c, rows_per, done);
+    case KIND_EVEN_FLOAT: return run_digit_prescan_scan<KIND_EVEN_FLOAT>(c, rows_per, done);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -503,8 +503,9 @@ gms_status multisplit_big_impl(const uint32_t* kin, const uint32_t* vin, uint32_
     c.scratch = base;
     c.bucket_bytes = base + make_geometry(n, c.logb, kv).off_buckets;
     c.stream = stream;
-    cudaError_t e = dispatch_digit_prescan(desc->kind, c, &c.rows_per);
-    if (e == cudaSuccess) e = run_digit_postscan(c);
+    bool done = false;
+    cudaError_t e = dispatch_digit_prescan(desc->kind, c, &c.rows_per, &done);
+    if (e == cudaSuccess && !done) e = run_digit_postscan(c);
     if (e != cudaSuccess) return cuda_status(e);
   }
   if (h_offsets == nullptr) return GMS_SUCCESS;

@@ -473,7 +473,10 @@ cudaError_t run_batch_class_t(const BatchClassLaunch& c, int stage) {
     auto kern = batch_postscan_kernel<C, KIND>;
     cudaError_t e = ensure_smem_limit(kern, smem, smem_done);
     if (e != cudaSuccess) return e;
-    kern<<<c.class_tiles, C::THREADS, smem, c.stream>>>(c.segs, c.tile_map, c.matrix, c.hdr, c.byte_area);
+    static std::atomic<int> per_sm{0};
+    const uint32_t wave = persistent_grid(kern, C::THREADS, c.class_tiles, per_sm, smem);
+    kern<<<c.class_tiles, C::THREADS, smem, c.stream>>>(c.segs, c.tile_map, c.matrix, c.hdr, c.byte_area,
+                                                        (GMS_PREFETCH_WAVES * wave) / 4u);
     return cudaGetLastError();
   }
 }
@@ -552,12 +555,16 @@ cudaError_t run_histogram(const uint32_t* keys, uint32_t n, int logb, const Buck
 
 // ------------------------------------------- more than 256 buckets
 template <int KIND, int LOGB, bool KV>
-cudaError_t digit_prescan_scan_t(const DigitPass& c, uint32_t* rows_per) {
+cudaError_t digit_prescan_scan_t(const DigitPass& c, uint32_t* rows_per, bool* done) {
   using S = TileShape<LOGB, KV>;
   using C = TileCfg<LOGB, S::WARPS, S::IPT, KV>;
   const Geometry g = make_geometry(c.n, LOGB, KV);
-  if (g.num_tiles == 0) return cudaSuccess;
+  *done = g.num_tiles == 0;
+  if (*done) return cudaSuccess;
   if (c.bucket_bytes == nullptr) return cudaErrorInvalidValue;
+  cudaError_t e = launch_fused<C, DigitPolicy<KIND, LOGB>>(c.kin, c.vin, c.kout, c.vout, c.n, c.bp, c.scratch,
+                                                           g.bytes_full, g, c.stream, nullptr, done);
+  if (e != cudaSuccess || *done) return e;
   auto* hdr = reinterpret_cast<ScratchHeader*>(c.scratch);
   auto* status = reinterpret_cast<uint64_t*>(c.scratch + g.off_status);
   auto* matrix = reinterpret_cast<uint32_t*>(c.scratch + g.off_matrix);
@@ -568,7 +575,7 @@ cudaError_t digit_prescan_scan_t(const DigitPass& c, uint32_t* rows_per) {
   *rows_per = rows != nullptr ? (g.num_tiles + grid - 1) / grid : 0u;
   kern<<<grid, C::THREADS, 0, c.stream>>>(c.kin, c.n, g.num_tiles, matrix, c.bp, hdr, status, g.num_chunks,
                                           c.bucket_bytes, *rows_per);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (rows != nullptr) return run_scan_rows(rows, C::B, g.num_tiles, *rows_per, status, hdr, c.stream);
   return run_scan(matrix, g.m, status, hdr, c.stream);
@@ -611,8 +618,8 @@ cudaError_t digit_postscan_t(const DigitPass& c) {
   }
 
 template <int KIND>
-cudaError_t run_digit_prescan_scan(const DigitPass& c, uint32_t* rows_per) {
-  GMS_DIGIT_SWITCH((c, rows_per), digit_prescan_scan_t, KIND,)
+cudaError_t run_digit_prescan_scan(const DigitPass& c, uint32_t* rows_per, bool* done) {
+  GMS_DIGIT_SWITCH((c, rows_per, done), digit_prescan_scan_t, KIND,)
 }
 
 template <int KIND>
@@ -660,7 +667,7 @@ cudaError_t run_big_offsets(const uint32_t* sorted_keys, uint32_t n, const Bucke
                                              int32_t*, cudaStream_t);
 
 #define GMS_INSTANTIATE_BIG(K)                                                           \
-  template cudaError_t gms::run_digit_prescan_scan<K>(const gms::DigitPass&, uint32_t*);           \
+  template cudaError_t gms::run_digit_prescan_scan<K>(const gms::DigitPass&, uint32_t*, bool*);           \
   template cudaError_t gms::run_big_histogram<K>(const uint32_t*, uint32_t, const gms::BucketParams&, uint32_t*, \
                                                  cudaStream_t);                                                 \
   template cudaError_t gms::run_big_offsets<K>(const uint32_t*, uint32_t, const gms::BucketParams&, uint32_t*, \

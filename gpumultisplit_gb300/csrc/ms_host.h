@@ -209,9 +209,10 @@ struct DigitPass {
 
 // Prescan (identifier evaluated, digit kept as a byte) and scan of a digit
 // pass; defined per kind in inst_big.cu.
-// *rows_per: the postscan's (DigitPass::rows_per).
+// *rows_per: the postscan's (DigitPass::rows_per).  *done: the pass ran whole, as
+// one launch.
 template <int KIND>
-cudaError_t run_digit_prescan_scan(const DigitPass& c, uint32_t* rows_per);
+cudaError_t run_digit_prescan_scan(const DigitPass& c, uint32_t* rows_per, bool* done);
 // Postscan of a digit pass from the bytes (inst_big_post.cu).
 cudaError_t run_digit_postscan(const DigitPass& c);
 // Adds the count of every whole bucket id in [0, p.num_buckets) into hist
