@@ -8,8 +8,8 @@
 // so a scanned offset is the segment's start within its scan group (`base`,
 // the sum of the n of earlier segments in the group) plus the offset inside
 // the segment; the postscan subtracts `base`.  Segments whose identifier is
-// costly (range, div, even-float) get a byte per key in the batch's byte
-// area: the prescan stores each key's bucket there and the postscan reads it.
+// costly (range; div and even-float for keys alone) get a byte per key in the
+// batch's byte area: the prescan stores each key's bucket there and the postscan reads it.
 #pragma once
 
 #include "multisplit_kernels.cuh"

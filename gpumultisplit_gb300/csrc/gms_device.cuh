@@ -546,10 +546,10 @@ __host__ __device__ constexpr uint32_t big_identifier_smem_words() {
 // Where splitter i lies in the shared area.  The second digit pass meets keys
 // whose ids agree modulo the first digit's width, so their splitters would
 // share a bank: its prescan of 16.8 M keys into 4096 buckets took 67 us, the
-// first pass's 49.  Few searches reach a splitter at all when there are not
-// more of them than cells, and the extra instructions cost more (300 buckets:
-// 187 us without, 191 with).
-__device__ __forceinline__ bool big_split_swizzled(uint32_t B) { return B > RANGE_LUT_CELLS; }
+// first pass's 49.  Elsewhere keys meet splitters at random and the extra
+// instructions only cost (histogram of 2^28 keys into 4096 bins: 0.81 ms
+// without, 0.88 with), as they do when there are not more splitters than cells
+// (300 buckets: 187 us without, 191 with).
 __device__ __forceinline__ uint32_t big_split_slot(uint32_t i, bool swizzled) {
   return swizzled ? i ^ ((i >> 5) & 31u) : i;
 }
@@ -569,7 +569,8 @@ __device__ __forceinline__ uint32_t big_upper_bound(const uint32_t* s_split, uin
 
 // The whole bucket id of a key, in [0, B).
 template <int KIND>
-__device__ __forceinline__ uint32_t big_bucket_id(uint32_t key, const BucketParams& p, const uint32_t* s_split) {
+__device__ __forceinline__ uint32_t big_bucket_id(uint32_t key, const BucketParams& p, const uint32_t* s_split,
+                                                  bool swizzled = false) {
   const uint32_t B = p.num_buckets;
   if constexpr (KIND == KIND_DELTA) {
     return __umulhi(key, B);
@@ -579,8 +580,8 @@ __device__ __forceinline__ uint32_t big_bucket_id(uint32_t key, const BucketPara
     return (key >> p.shift) & (B - 1);
   } else if constexpr (KIND == KIND_RANGE) {
     const uint32_t e = s_split[GMS_RANGE_BIG_MAX + (key >> (32 - RANGE_LUT_BITS))];
-    const uint32_t c = big_split_swizzled(B) ? big_upper_bound<true>(s_split, key, e & 0xFFFFu, e >> 16)
-                                             : big_upper_bound<false>(s_split, key, e & 0xFFFFu, e >> 16);
+    const uint32_t c = swizzled ? big_upper_bound<true>(s_split, key, e & 0xFFFFu, e >> 16)
+                                : big_upper_bound<false>(s_split, key, e & 0xFFFFu, e >> 16);
     return c == 0u ? B - 1u : c - 1u;
   } else if constexpr (KIND == KIND_MASK) {
     return (key & p.param) ? 1u : 0u;
@@ -593,13 +594,13 @@ __device__ __forceinline__ uint32_t big_bucket_id(uint32_t key, const BucketPara
 // Fill the full identifier's shared area (RANGE: B splitters and the table).
 // All threads call; a barrier must follow.
 template <int KIND>
-__device__ __forceinline__ void prepare_big_identifier(uint32_t* s_split, const BucketParams& p) {
+__device__ __forceinline__ void prepare_big_identifier(uint32_t* s_split, const BucketParams& p,
+                                                       bool swizzled = false) {
   if constexpr (KIND == KIND_RANGE) {
     // Loads eight deep (one at a time they took 10 of the 17 us that a block
     // spent here for 4096 splitters), then for each thread one search over all
     // splitters for its first cell and one from there for each cell's end.
     const uint32_t B = p.num_buckets;
-    const bool swizzled = big_split_swizzled(B);
     for (uint32_t i0 = threadIdx.x; i0 < B; i0 += 8u * blockDim.x) {
       uint32_t v[8];
 #pragma unroll
@@ -639,13 +640,17 @@ __device__ __forceinline__ void prepare_big_identifier(uint32_t* s_split, const 
   }
 }
 
+// Whether a digit pass spreads its splitters over the banks (big_split_slot).
+__device__ __forceinline__ bool digit_swizzles(const BucketParamsBig& p) {
+  return p.digit_shift != 0u && p.base.num_buckets > RANGE_LUT_CELLS;
+}
+
 template <int KIND, int LOGB>
 struct DigitId {
-  BucketParams p;
-  uint32_t shift;
+  BucketParamsBig p;
   const uint32_t* s_split;
   __device__ __forceinline__ uint32_t operator()(uint32_t key) const {
-    return (big_bucket_id<KIND>(key, p, s_split) >> shift) & ((1u << LOGB) - 1u);
+    return (big_bucket_id<KIND>(key, p.base, s_split, digit_swizzles(p)) >> p.digit_shift) & ((1u << LOGB) - 1u);
   }
 };
 
@@ -660,9 +665,9 @@ struct DigitPolicy {
   static constexpr bool USES_SMEM = KIND == KIND_RANGE;
   static constexpr uint32_t SMEM_WORDS = big_identifier_smem_words<KIND>();
   __device__ __forceinline__ static void prepare(uint32_t* s, const Params& p) {
-    prepare_big_identifier<KIND>(s, p.base);
+    prepare_big_identifier<KIND>(s, p.base, digit_swizzles(p));
   }
-  __device__ __forceinline__ static Id make(const Params& p, const uint32_t* s) { return Id{p.base, p.digit_shift, s}; }
+  __device__ __forceinline__ static Id make(const Params& p, const uint32_t* s) { return Id{p, s}; }
 };
 
 // The postscan of a digit pass reads the prescan's bytes only; one policy

@@ -350,8 +350,8 @@ int device_sm_count();
 // ping-pong buffers, exactly as the multisplit passes would.
 constexpr int kOnesweepMaxPasses = 8;
 // Sorts of at least this many keys take the one-sweep passes by default
-// (none: on GB300 they measured slower than the multisplit passes, 7.4 against
-// 5.6 ms for 2^28 pairs with 7-bit digits).
+// (none: on GB300 they measured slower than the multisplit passes, 6.4 against
+// 4.9 ms for 2^28 pairs with 7-bit digits).
 constexpr uint32_t kOnesweepMinKeys = 0xFFFFFFFFu;
 size_t onesweep_scratch_bytes(uint32_t n, int passes, const uint32_t* logb);
 cudaError_t run_onesweep_sort(const uint32_t* kin, uint32_t* kout, const uint32_t* vin, uint32_t* vout, uint32_t n,

@@ -105,10 +105,10 @@ gms_status gms_read_device_error(const void* d_scratch, uint32_t* h_code, gms_st
 /* ------------------------------------------------------------ multisplit */
 /* Replaces multisplit_allocate_key_only / _key_value (src/api/multisplit.cuh:50-74):
  * scratch bytes for calls with n <= max_elements.  The size includes one byte
- * per key that identifiers costly to evaluate (range, div, even-float) use to
- * evaluate the identifier once instead of twice; a scratch without that room
- * (max_elements bytes less, rounded up to 256) still works, more slowly for
- * those identifiers. */
+ * per key, in which identifiers costly to evaluate (range; div and even-float
+ * for keys alone) keep their buckets and small calls their counts, and, from 65
+ * buckets up, a second copy of the count matrix as rows.  A scratch without
+ * that room (down to the matrix and the scan's state) still works, more slowly. */
 gms_status gms_multisplit_scratch_bytes(uint32_t max_elements, uint32_t num_buckets, int key_value,
                                         size_t* bytes);
 
@@ -188,6 +188,9 @@ gms_status gms_sort_7bit_key_value(const uint32_t* d_key_in, uint32_t* d_key_out
  * src/api/multisplit_sort_pairs.cuh:67-260), same schedules:
  *   4: eight 4-bit passes;  5: six 5-bit passes then bits [30,32);
  *   6: 4-bit, 4-bit, then four 6-bit passes;  7: as above;  8: four 8-bit passes.
+ * Under GMS_SORT_AUTO a sort of up to 2.5 M keys runs as one launch, in 8-bit
+ * digits whatever the width; the sorted order is the same.  The reported size
+ * then includes its counts (at most 0.6 MB); without them the passes run.
  * digit_bits outside 4..8 is GMS_ERROR_INVALID_VALUE. */
 gms_status gms_sort_scratch_bytes(uint32_t max_elements, int digit_bits, int key_value, size_t* bytes);
 gms_status gms_sort_key_only(const uint32_t* d_key_in, uint32_t* d_key_out, uint32_t n, int digit_bits,
