@@ -53,9 +53,11 @@ struct TileCfg {
   static constexpr uint32_t WB = B < 32 ? 32 : B;  // row width of the per-warp count table
   // Ranks by shared-memory atomics (postscan_tile); by ballots at the smallest
   // bucket counts, where few ballots suffice and many lanes meet in a counter.
-  // At 2^28, ballots / atomics: pairs 16 buckets 0.893 / 0.866 ms, 32 buckets
-  // 0.955 / 0.867; keys 16 buckets 0.694 / 0.725, 32 buckets 0.770 / 0.712.
-  static constexpr bool ATOMIC = LOGB_ >= (KV_ ? 4 : 5);
+  // At 2^28, ballots / atomics: keys 16 buckets 0.694 / 0.725 ms, 32 buckets
+  // 0.770 / 0.692; pairs 32 buckets 0.955 / 0.874.  Pairs into 16 buckets gain
+  // on uniform keys (0.893 / 0.866) but lose on skewed ones (2^25 Zipf pairs
+  // 123 / 128 us, four of the buckets 121 / 142).
+  static constexpr bool ATOMIC = LOGB_ >= 5;
 
   static_assert(IPT % 4 == 0, "IPT must be a multiple of 4 (16-byte vector loads)");
   static_assert(TILE <= 65536, "in-tile positions are packed into 16 bits");
@@ -500,9 +502,8 @@ __device__ __forceinline__ uint32_t peers_by_ballot(uint32_t b) {
 }
 
 // Lanes of a warp's first slot in one bucket from which on the warp treats its
-// most frequent buckets apart (with few buckets a crowd is no sign of skew).
-// 33.5 M Zipf pairs into 16 buckets took 130 us at 8 lanes and 122 at 12; keys
-// in four of 128 buckets 167 at 8 and 209 at 12.
+// most frequent buckets apart (with 32 buckets a crowd of 8 is no sign of skew:
+// 2^25 Zipf pairs took 130 us at 8 lanes and 124 at 12).
 __host__ __device__ constexpr uint32_t rank_crowd(int logb) { return logb <= 5 ? 12u : 8u; }
 
 // Where a tile's global bucket offsets come from.  Thread b < B holds the
@@ -635,8 +636,8 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
     for (int j = 0; j < IPT; ++j) packed[j] = bucket_at(wbase + uint32_t(j) * 32u + lane) << 16;
     // Lanes that meet in a counter are served one after another, so a warp
     // whose first slot is crowded takes its two most frequent buckets by one
-    // ballot each, their counts in registers; if a third is crowded too, all
-    // buckets go by ballots.
+    // ballot each, their counts in registers; if a third is crowded too, four
+    // (32 lanes have no room for a fifth crowd).
     const uint32_t b0 = packed[0] >> 16;
     const uint32_t peers0 =
         FULL ? peers_by_ballot<LOGB>(b0) : peers_by_ballot<LOGB>(b0) & __ballot_sync(~0u, wbase + lane < cnt);
@@ -649,45 +650,46 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
         if (FULL || pos < cnt) packed[j] |= atomicAdd(wh + (packed[j] >> 16), 1u);
       }
     } else {
-      const uint32_t d1 = most & 0xFFFFu;
-      const uint32_t next = __reduce_max_sync(~0u, b0 == d1 ? 0u : crowd);
-      const uint32_t d2 = next != 0u ? next & 0xFFFFu : 0xFFFFu;
-      const uint32_t third = __reduce_max_sync(~0u, b0 == d1 || b0 == d2 ? 0u : crowd);
-      if ((third >> 16) < rank_crowd(LOGB)) {
-        uint32_t run1 = 0, run2 = 0;
+      // Ranks with the D most frequent buckets d[] (0xFFFF: none) taken by ballots.
+      auto rank_apart = [&](auto count, const uint32_t* d) {
+        constexpr int D = decltype(count)::value;
+        uint32_t run[D];
+#pragma unroll
+        for (int i = 0; i < D; ++i) run[i] = 0;
 #pragma unroll
         for (int j = 0; j < IPT; ++j) {
           const bool valid = FULL || wbase + uint32_t(j) * 32u + lane < cnt;
           const uint32_t b = packed[j] >> 16;
-          const uint32_t m1 = __ballot_sync(~0u, valid && b == d1), m2 = __ballot_sync(~0u, valid && b == d2);
-          if (b == d1)
-            packed[j] |= run1 + __popc(m1 & lt);
-          else if (b == d2)
-            packed[j] |= run2 + __popc(m2 & lt);
-          else if (valid)
-            packed[j] |= atomicAdd(wh + b, 1u);
-          run1 += __popc(m1);
-          run2 += __popc(m2);
-        }
-        if (lane == 0) {
-          wh[d1] = run1;
-          if (d2 < B) wh[d2] = run2;
-        }
-      } else {
+          bool apart = !valid;
 #pragma unroll
-        for (int j = 0; j < IPT; ++j) {
-          const bool valid = FULL || wbase + uint32_t(j) * 32u + lane < cnt;
-          const uint32_t b = packed[j] >> 16;
-          uint32_t peers = peers_by_ballot<LOGB>(b);
-          if (!FULL) peers &= __ballot_sync(~0u, valid);
-          const uint32_t rank = __popc(peers & lt);
-          const uint32_t before = wh[b];
-          __syncwarp();
-          if (valid && rank == 0) wh[b] = before + __popc(peers);
-          __syncwarp();
-          packed[j] |= before + rank;
+          for (int i = 0; i < D; ++i) {
+            const bool mine = valid && b == d[i];
+            const uint32_t m = __ballot_sync(~0u, mine);
+            if (mine) packed[j] |= run[i] + __popc(m & lt);
+            apart |= mine;
+            run[i] += __popc(m);
+          }
+          if (!apart) packed[j] |= atomicAdd(wh + b, 1u);
         }
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+          if (lane == 0 && d[i] < B) wh[d[i]] = run[i];
+        }
+      };
+      uint32_t d[4];
+      d[0] = most & 0xFFFFu;
+      uint32_t left = b0 == d[0] ? 0u : crowd;
+#pragma unroll
+      for (int i = 1; i < 4; ++i) {
+        const uint32_t next = __reduce_max_sync(~0u, left);
+        d[i] = next != 0u ? next & 0xFFFFu : 0xFFFFu;
+        if (b0 == d[i]) left = 0u;
+        if (i == 2 && (next >> 16) < rank_crowd(LOGB)) d[2] = 0xFFFFu;  // no third crowd: two suffice
       }
+      if (d[2] == 0xFFFFu)
+        rank_apart(std::integral_constant<int, 2>{}, d);
+      else
+        rank_apart(std::integral_constant<int, 4>{}, d);
     }
   } else {
     // Lane l counts bucket l: its mask of lanes holding bucket l comes straight
