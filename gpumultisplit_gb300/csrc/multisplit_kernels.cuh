@@ -610,12 +610,14 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
 
   // ---- 1. stable in-warp ranks
   const typename P::Id ident = P::make(bp, s_split);
-  // Bucket of the staged key at in-tile position pos.
+  // Bucket of the staged key at in-tile position pos; 0 past a partial tile's
+  // keys, where shared memory holds anything: a caller's functor may look its
+  // key up in memory, so it is evaluated on the input's keys only.
   auto bucket_at = [&](uint32_t pos) -> uint32_t {
     if constexpr (GIVEN)
       return uint32_t(s_rb[pos]) & (B - 1);
     else
-      return ident(s_k[pos]);
+      return FULL || pos < cnt ? ident(s_k[pos]) : 0u;
   };
   uint32_t packed[IPT];  // (bucket << 16) | rank among same-bucket keys of this warp
   const uint32_t wbase = warp * (IPT * 32u);
