@@ -271,6 +271,9 @@ __device__ __forceinline__ void fused_tile(const typename C::KT* kin, const type
   if (tid == 0) *reinterpret_cast<uint32_t*>(smem + L::OFF_FLAG) = 0u;
   KT* s_k = reinterpret_cast<KT*>(smem + L::OFF_K);
   stage_tile<C::THREADS, C::IPT>(s_k, kin + base, cnt);
+  if constexpr (!P::ANY_KEY) {
+    if (cnt == 0 && tid == 0) s_k[0] = __ldcg(kin);  // postscan_tile evaluates the identifier on it
+  }
   if constexpr (C::KV) stage_tile<C::THREADS, C::IPT>(reinterpret_cast<VT*>(smem + L::OFF_V), vin + base, cnt);
   uint32_t* s_state = GIVEN ? s_ident : reinterpret_cast<uint32_t*>(smem + L::OFF_SPLIT);
   P::prepare(s_state, bp);
@@ -340,6 +343,7 @@ struct FieldPolicy {
   template <bool KV>
   static constexpr bool CHEAP = CHEAP_;
   static constexpr bool USES_SMEM = false;
+  static constexpr bool ANY_KEY = true;
   static constexpr uint32_t SMEM_WORDS = 1;
   __device__ __forceinline__ static void prepare(uint32_t*, const Params&) {}
   __device__ __forceinline__ static Id make(const Params& p, const uint32_t*) { return Id{p}; }

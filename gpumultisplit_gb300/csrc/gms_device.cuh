@@ -397,6 +397,7 @@ __host__ __device__ constexpr bool kind_keeps_bucket_bytes(int kind, bool kv) {
 // identifier.  DescPolicy covers the precompiled descriptor kinds; the drop-in
 // C++ headers use FunctorPolicy to instantiate the same kernels with any
 // device-callable functor, compiled in the caller's translation unit.
+// ANY_KEY: the identifier may be evaluated on words that are not the input's keys.
 template <int KIND, int LOGB>
 struct DescPolicy {
   using Params = BucketParams;
@@ -404,6 +405,7 @@ struct DescPolicy {
   template <bool KV>
   static constexpr bool CHEAP = !kind_keeps_bucket_bytes(KIND, KV);
   static constexpr bool USES_SMEM = KIND == KIND_RANGE;
+  static constexpr bool ANY_KEY = true;
   static constexpr uint32_t SMEM_WORDS = identifier_smem_words<KIND, LOGB>();
   __device__ __forceinline__ static void prepare(uint32_t* s, const Params& p) { prepare_identifier<KIND, LOGB>(s, p); }
   __device__ __forceinline__ static Id make(const Params& p, const uint32_t* s) { return Id{p, s}; }
@@ -512,6 +514,7 @@ struct DescPolicy64 {
   template <bool KV>
   static constexpr bool CHEAP = false;  // 64-bit keys always keep their buckets as bytes
   static constexpr bool USES_SMEM = KIND == KIND_RANGE;
+  static constexpr bool ANY_KEY = true;
   static constexpr uint32_t SMEM_WORDS = identifier64_smem_words<KIND, LOGB>();
   __device__ __forceinline__ static void prepare(uint32_t* s, const Params& p) {
     prepare_identifier64<KIND, LOGB>(s, p);
@@ -663,6 +666,7 @@ struct DigitPolicy {
   template <bool KV>
   static constexpr bool CHEAP = false;
   static constexpr bool USES_SMEM = KIND == KIND_RANGE;
+  static constexpr bool ANY_KEY = true;
   static constexpr uint32_t SMEM_WORDS = big_identifier_smem_words<KIND>();
   __device__ __forceinline__ static void prepare(uint32_t* s, const Params& p) {
     prepare_big_identifier<KIND>(s, p.base, digit_swizzles(p));
@@ -681,6 +685,7 @@ struct GivenBytesPolicy {
   template <bool KV>
   static constexpr bool CHEAP = false;
   static constexpr bool USES_SMEM = false;
+  static constexpr bool ANY_KEY = true;
   static constexpr uint32_t SMEM_WORDS = 1;
   __device__ __forceinline__ static void prepare(uint32_t*, const Params&) {}
   __device__ __forceinline__ static Id make(const Params&, const uint32_t*) { return Id{}; }
@@ -703,6 +708,7 @@ struct FunctorPolicy {
   template <bool KV>
   static constexpr bool CHEAP = false;  // cost unknown: buckets are computed once per key and kept
   static constexpr bool USES_SMEM = false;
+  static constexpr bool ANY_KEY = false;  // it may look its key up in memory
   static constexpr uint32_t SMEM_WORDS = 1;
   __device__ __forceinline__ static void prepare(uint32_t*, const Params&) {}
   __device__ __forceinline__ static Id make(const Params& f, const uint32_t*) { return Id{f}; }

@@ -579,7 +579,8 @@ __device__ __forceinline__ void rows_to_matrix(const uint32_t* __restrict__ rows
 //
 // GIVEN: the tile's buckets were staged as bytes at the bucket-byte area (in
 // input order) by the caller, so the identifier is not evaluated; phase 3
-// overwrites that area with the buckets in sorted order.
+// overwrites that area with the buckets in sorted order.  Else, unless P::ANY_KEY,
+// position 0 holds one of the input's keys even if the tile is empty.
 //
 // STREAM_HINTS: the output stores mark their L2 lines evict-first (the batch
 // queue keeps keys that are read twice in L2 meanwhile; 32-bit elements).
@@ -610,14 +611,16 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
 
   // ---- 1. stable in-warp ranks
   const typename P::Id ident = P::make(bp, s_split);
-  // Bucket of the staged key at in-tile position pos; 0 past a partial tile's
-  // keys, where shared memory holds anything: a caller's functor may look its
-  // key up in memory, so it is evaluated on the input's keys only.
+  // Bucket of the staged key at in-tile position pos.  Past a partial tile's keys
+  // shared memory holds anything: where the identifier is not to see that, those
+  // slots take position 0's key.  (A branch around each evaluation kept a warp's
+  // searches from overlapping: 10007 range pairs 8.4 -> 10.3 us; and the clamp
+  // costs the key-only kernel into 32 buckets a spill, 2 % of a 5-bit sort.)
   auto bucket_at = [&](uint32_t pos) -> uint32_t {
     if constexpr (GIVEN)
       return uint32_t(s_rb[pos]) & (B - 1);
     else
-      return FULL || pos < cnt ? ident(s_k[pos]) : 0u;
+      return ident(s_k[FULL || P::ANY_KEY || pos < cnt ? pos : 0u]);
   };
   uint32_t packed[IPT];  // (bucket << 16) | rank among same-bucket keys of this warp
   const uint32_t wbase = warp * (IPT * 32u);

@@ -49,9 +49,9 @@ int main() {
           multisplit_key_only(keys, ko, n, ctx, f);
         return multisplit_last_error();
       };
-      // One tile, one cluster, a grid, three stages; each with the reported
+      // One tile, clusters without and with an empty block, a grid, three stages; each with the reported
       // scratch and with the smallest that is taken (no byte per key).
-      for (uint32_t n : {1u, 33u, TILE + 1, 20 * TILE + 1, MOST}) {
+      for (uint32_t n : {1u, 33u, TILE + 1, 2 * TILE + 1, 20 * TILE + 1, MOST}) {
         for (bool small : {false, true}) {
           ctx.temp_storage_bytes = most_bytes;
           bad += run(large, 600 * TILE, 0) != GMS_SUCCESS;
