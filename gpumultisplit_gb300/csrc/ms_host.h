@@ -87,7 +87,7 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // rows: 2^25 keys 64 buckets 102 / 102, 128 116 / 109, 256 148 / 123; pairs 32
 // buckets 116 / 121, 64 125 / 127, 128 138 / 137, 256 183 / 165), and from 512
 // tiles up; fewer run as one launch where they can, and over the matrix where not.
-constexpr bool counts_as_rows(int logb, uint32_t num_tiles) { return logb >= 7 && num_tiles >= 512; }
+constexpr bool counts_as_rows(int logb, uint32_t num_tiles) { return logb >= ROWS_MIN_LOGB && num_tiles >= 512; }
 
 // Scratch layout of one multisplit: [header 256 B][count matrix u32 x B*tiles][scan status u64 x chunks].
 // The matrix always starts at byte 256, whatever n is.
