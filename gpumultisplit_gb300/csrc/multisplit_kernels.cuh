@@ -238,10 +238,16 @@ __device__ __forceinline__ void count_tiles(const uint32_t* __restrict__ keys, u
 // bucket is also stored there as one byte, so the postscan need not evaluate
 // the identifier again.
 //
-// Each block counts a contiguous run of tiles, as even as whole tiles allow, and keeps the counts of
-// PRESCAN_GROUP consecutive tiles in shared memory, then writes them bucket by
-// bucket: a warp stores whole runs of consecutive matrix words (the matrix is
-// bucket-major) instead of one scattered word per bucket and tile.
+// Each block counts a contiguous run of tiles, ceil(tiles / blocks) of them, and
+// keeps the counts of PRESCAN_GROUP tiles in shared memory, then writes them
+// bucket by bucket: a warp stores whole runs of consecutive matrix words (the
+// matrix is bucket-major) instead of one scattered word per bucket and tile.
+// In ranges of at least two groups the groups are those of the matrix, [8 g,
+// 8 g + 8), wherever a range begins: groups counted from a range's own start
+// write every sector in two parts, which leave L2 separately once the matrix is
+// large (256 buckets, us, groups of the range / of the matrix: 2^27 keys 96 / 92,
+// 2^28 208 / 183, 2^30 855 / 723).  Shorter ranges count from their start: the
+// matrix's groups would cut them in two (2^24 keys 16.9 / 18.4).
 //
 // rows_per != 0 (the one-call path): the counts go into rows instead,
 // counts[tile * B + b], one coalesced store per tile.  A block's range is then
@@ -254,6 +260,25 @@ __device__ __forceinline__ void count_tiles(const uint32_t* __restrict__ keys, u
 // all counts.
 constexpr uint32_t PRESCAN_GROUP = 8;
 
+// Tiles of a prescan block's range.  whole_groups: a multiple of the group where
+// that lengthens the range by at most a sixteenth, so that no two blocks write
+// to one sector.
+__host__ __device__ inline uint32_t prescan_tiles_per_block(uint32_t num_tiles, uint32_t blocks, bool whole_groups) {
+  const uint32_t per = (num_tiles + blocks - 1) / blocks;
+  const uint32_t whole = (per + PRESCAN_GROUP - 1) / PRESCAN_GROUP * PRESCAN_GROUP;
+  return whole_groups && (whole - per) * 16u <= per ? whole : per;
+}
+
+// Where ranges of whole groups pay: with identifiers that leave the prescan bound
+// by memory (us, any range / whole groups: 256 buckets 2^28 keys 183 / 178, 2^30
+// 723 / 695; 190 M keys, ranges of 62 / 64 tiles: 16 buckets 128 / 115, 64 130 /
+// 115, 128 135 / 118).  A splitter search is bound by its longest range (256
+// buckets, 2^28 keys 330 / 340).
+template <class P>
+constexpr bool prescan_whole_groups() {
+  return !P::USES_SMEM;
+}
+
 template <class C>
 struct PrescanCounts {
   static constexpr uint32_t B = C::B;
@@ -261,14 +286,17 @@ struct PrescanCounts {
   uint32_t* counts;
   uint32_t* s_cnt;  // B * G words
   uint32_t num_tiles, first, last;
+  uint32_t origin;  // where groups are counted from
   bool rows;
   uint32_t run;     // rows: count of bucket tid in the range so far
 
-  __device__ __forceinline__ PrescanCounts(uint32_t* counts_, uint32_t* s_cnt_, uint32_t num_tiles_, uint32_t rows_per)
+  __device__ __forceinline__ PrescanCounts(uint32_t* counts_, uint32_t* s_cnt_, uint32_t num_tiles_, uint32_t rows_per,
+                                           bool whole_groups)
       : counts(counts_), s_cnt(s_cnt_), num_tiles(num_tiles_), rows(rows_per != 0), run(0) {
-    const uint32_t per = rows ? rows_per : (num_tiles + gridDim.x - 1) / gridDim.x;
+    const uint32_t per = rows ? rows_per : prescan_tiles_per_block(num_tiles, gridDim.x, whole_groups);
     first = min(blockIdx.x * per, num_tiles);
     last = min(first + per, num_tiles);
+    origin = per < 2 * G ? first : 0u;
   }
   // Called by all threads after each tile; thread tid < B has the tile's count of bucket tid.
   __device__ __forceinline__ void done(uint32_t tile, uint32_t total) {
@@ -281,14 +309,14 @@ struct PrescanCounts {
       }
       return;
     }
-    const uint32_t g = (tile - first) % G;
+    const uint32_t g = (tile - origin) % G;
     if (tid < B) s_cnt[tid * G + g] = total;
     if (g == G - 1 || tile + 1 == last) {
       const uint32_t group_first = tile - g;
       __syncthreads();
       for (uint32_t i = tid; i < B * G; i += C::THREADS) {
         const uint32_t t = group_first + i % G;
-        if (t < last) counts[(i / G) * num_tiles + t] = s_cnt[i];
+        if (t >= first && t < last) counts[(i / G) * num_tiles + t] = s_cnt[i];
       }
       __syncthreads();
     }
@@ -323,7 +351,7 @@ __global__ void __launch_bounds__(C::THREADS) prescan_kernel(const uint32_t* __r
   Counter counter(P::make(bp, s_split), s_hist);
   counter.clear_shared();
   __syncthreads();
-  PrescanCounts<C> out(counts, s_cnt, num_tiles, rows_per);
+  PrescanCounts<C> out(counts, s_cnt, num_tiles, rows_per, prescan_whole_groups<P>());
   auto done = [&](uint32_t tile) { out.done(tile, counter.block_total()); };
   if constexpr (!P::template CHEAP<C::KV>) {
     if (bucket_bytes != nullptr) {
@@ -377,7 +405,7 @@ __global__ void __launch_bounds__(C::THREADS) prescan64_kernel(const uint64_t* _
   Counter counter(P::make(bp, s_split), s_hist);
   counter.clear_shared();
   __syncthreads();
-  PrescanCounts<C> out(counts, s_cnt, num_tiles, rows_per);
+  PrescanCounts<C> out(counts, s_cnt, num_tiles, rows_per, prescan_whole_groups<P>());
   const uint32_t first = out.first, last = out.last;
   const bool vec_ok = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
   const uint32_t full_tiles = vec_ok ? min(n / TILE, last) : 0u;
