@@ -5,6 +5,7 @@
 #include <cstring>
 
 #include "../../include/gpumultisplit.h"
+#include "host_starts.h"
 #include "ms_host.h"
 #include "scan_kernels.cuh"
 
@@ -84,37 +85,57 @@ bool overlaps(const void* a, const void* b, uint32_t n, size_t elem_a = 4, size_
   return x < y + uintptr_t(n) * elem_b && y < x + uintptr_t(n) * elem_a;
 }
 
-// Where a call's last kernel leaves the bucket starts for the host: 256 words
-// of pinned memory per calling thread, allocated on its first call that asks
-// for offsets and freed when the thread ends.  Such a call waits for its stream
-// before it returns, so a thread's words serve one call at a time.  Against a
-// strided device-to-host copy of column 0 after the kernels, a call of 10 k
-// pairs at 32 buckets took 19 us instead of 24, without the copy's own latency.
-class HostStarts {
- public:
-  ~HostStarts() {
-    if (words_ != nullptr) cudaFreeHost(words_);
-  }
-  // null when pinned memory cannot be had (the caller then copies the matrix).
-  uint32_t* get() {
-    if (words_ == nullptr &&
-        cudaHostAlloc(reinterpret_cast<void**>(&words_), 256 * sizeof(uint32_t),
-                      cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-      cudaGetLastError();
-      words_ = nullptr;
-    }
-    return words_;
-  }
+uint32_t* alloc_pinned_words(size_t words) {
+  uint32_t* p = nullptr;
+  if (cudaHostAlloc(reinterpret_cast<void**>(&p), words * sizeof(uint32_t),
+                    cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess)
+    return p;
+  cudaGetLastError();
+  return nullptr;
+}
 
- private:
-  uint32_t* words_ = nullptr;
-};
-thread_local HostStarts t_starts;
+// A number of the current context that no later context of the process gets, or
+// 0 when it cannot be had.
+uint64_t current_context_id() {
+  using CtxGetId = int (*)(void* ctx, unsigned long long* id);  // cuCtxGetId
+  static const CtxGetId get_id = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<CtxGetId>(f);
+  }();
+  if (get_id == nullptr) return 0;
+  unsigned long long id = 0;
+  if (get_id(nullptr, &id) == 0) return id + 1;
+  // A thread's first call: make its device's primary context current.
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess || get_id(nullptr, &id) != 0) {
+    cudaGetLastError();
+    return 0;
+  }
+  return id + 1;
+}
+
+// The calling thread's pinned words for a call that returns bucket starts, or
+// null (the caller then copies the matrix).  Against a strided device-to-host
+// copy of column 0 after the kernels, a call of 10 k pairs at 32 buckets took 19
+// us instead of 24, without the copy's own latency.
+uint32_t* thread_starts() {
+  static StartsPool& pool = *new StartsPool(alloc_pinned_words);  // outlives every thread
+  thread_local ThreadStarts mine(pool);
+  return mine.get(current_context_id());
+}
 
 // Shared body of the multisplit entry points (stage mask selects the kernels).
+// starts (or null): receives the words in which the last kernel leaves the
+// bucket starts, if it does.
 gms_status multisplit_impl(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, uint32_t n,
                            const gms_bucket_desc* desc, bool kv, void* scratch, size_t scratch_bytes,
-                           int stages, cudaStream_t stream, uint32_t* starts = nullptr, bool keep_matrix = true) {
+                           int stages, cudaStream_t stream, uint32_t** starts = nullptr, bool keep_matrix = true) {
   int logb = 0;
   gms_status st = check_desc(desc, &logb);
   if (st != GMS_SUCCESS) return st;
@@ -140,7 +161,7 @@ gms_status multisplit_impl(const uint32_t* kin, const uint32_t* vin, uint32_t* k
   c.scratch = static_cast<unsigned char*>(scratch);
   c.stream = stream;
   c.scratch_bytes = scratch_bytes;
-  c.starts = starts;
+  if (starts != nullptr) c.starts = *starts = thread_starts();
   c.keep_matrix = keep_matrix;
   // Costly identifiers are evaluated once when the scratch has room for a
   // bucket byte per key (the prescan stores them, the postscan reads them).
@@ -149,7 +170,7 @@ gms_status multisplit_impl(const uint32_t* kin, const uint32_t* vin, uint32_t* k
 }
 
 // Bucket start offsets: matrix[b * num_tiles] for b < B (src/api/multisplit.cuh:143-149).
-// starts: the call's pinned words (HostStarts), or null.
+// starts: the call's pinned words, or null.
 gms_status copy_offsets(const void* scratch, uint32_t n, int logb, uint32_t B, bool kv, uint32_t* h_offsets,
                         cudaStream_t stream, const uint32_t* starts, int kw = 1, int vw = 1) {
   if (n == 0) {
@@ -367,9 +388,9 @@ gms_status compaction_impl(const uint32_t* kin, const uint32_t* vin, uint32_t* k
                            const gms_bucket_desc* desc, bool kv, void* scratch, size_t scratch_bytes,
                            uint32_t* h_num0, cudaStream_t stream) {
   if (desc == nullptr || desc->num_buckets != 2) return GMS_ERROR_INVALID_VALUE;
-  uint32_t* starts = h_num0 != nullptr && n != 0 ? t_starts.get() : nullptr;
-  gms_status st = multisplit_impl(kin, vin, kout, vout, n, desc, kv, scratch, scratch_bytes, STAGE_ALL, stream, starts,
-                                  h_num0 != nullptr && starts == nullptr);
+  uint32_t* starts = nullptr;
+  gms_status st = multisplit_impl(kin, vin, kout, vout, n, desc, kv, scratch, scratch_bytes, STAGE_ALL, stream,
+                                  h_num0 != nullptr ? &starts : nullptr);
   if (st != GMS_SUCCESS || h_num0 == nullptr) return st;
   // Start of bucket 1 = number of bucket-0 keys (multisplit2_compaction.cuh:541-542).
   uint32_t offsets[2];
@@ -590,7 +611,7 @@ size_t wide_required_bytes(const Geometry& g, int key_bytes) { return key_bytes 
 // 32-bit path; everything else the 64-bit instances.
 gms_status multisplit_wide_impl(const void* kin, const void* vin, void* kout, void* vout, uint32_t n, int key_bytes,
                                 int value_bytes, const gms_bucket_desc64* desc, void* scratch, size_t scratch_bytes,
-                                cudaStream_t stream, uint32_t* starts = nullptr, bool keep_matrix = false) {
+                                cudaStream_t stream, uint32_t** starts = nullptr) {
   if (!valid_widths(key_bytes, value_bytes)) return GMS_ERROR_INVALID_VALUE;
   const bool kv = value_bytes != 0;
   if (key_bytes == 4 && value_bytes != 8) {
@@ -635,8 +656,8 @@ gms_status multisplit_wide_impl(const void* kin, const void* vin, void* kout, vo
   c.scratch = static_cast<unsigned char*>(scratch);
   c.stream = stream;
   c.scratch_bytes = scratch_bytes;
-  c.starts = starts;
-  c.keep_matrix = keep_matrix;
+  if (starts != nullptr) c.starts = *starts = thread_starts();
+  c.keep_matrix = starts != nullptr && c.starts == nullptr;  // the offsets then come from it
   if (key_bytes == 8) {
     c.bp64 = to_params64(desc);
     c.bucket_bytes = c.scratch + g.off_buckets;
@@ -828,9 +849,9 @@ gms_status gms_multisplit_key_only(const uint32_t* d_key_in, uint32_t* d_key_out
   if (is_big(desc))
     return multisplit_big_impl(d_key_in, nullptr, d_key_out, nullptr, n, desc, false, d_scratch, scratch_bytes,
                                h_offsets, stream);
-  uint32_t* starts = h_offsets != nullptr && n != 0 ? t_starts.get() : nullptr;
+  uint32_t* starts = nullptr;
   gms_status st = multisplit_impl(d_key_in, nullptr, d_key_out, nullptr, n, desc, false, d_scratch, scratch_bytes,
-                                  STAGE_ALL, stream, starts);
+                                  STAGE_ALL, stream, h_offsets != nullptr ? &starts : nullptr);
   if (st != GMS_SUCCESS || h_offsets == nullptr) return st;
   int logb = 0;
   valid_buckets(desc->num_buckets, &logb);
@@ -844,9 +865,9 @@ gms_status gms_multisplit_key_value(const uint32_t* d_key_in, const uint32_t* d_
   if (is_big(desc))
     return multisplit_big_impl(d_key_in, d_value_in, d_key_out, d_value_out, n, desc, true, d_scratch,
                                scratch_bytes, h_offsets, stream);
-  uint32_t* starts = h_offsets != nullptr && n != 0 ? t_starts.get() : nullptr;
+  uint32_t* starts = nullptr;
   gms_status st = multisplit_impl(d_key_in, d_value_in, d_key_out, d_value_out, n, desc, true, d_scratch,
-                                  scratch_bytes, STAGE_ALL, stream, starts);
+                                  scratch_bytes, STAGE_ALL, stream, h_offsets != nullptr ? &starts : nullptr);
   if (st != GMS_SUCCESS || h_offsets == nullptr) return st;
   int logb = 0;
   valid_buckets(desc->num_buckets, &logb);
@@ -1016,10 +1037,9 @@ gms_status gms_multisplit_wide_scratch_bytes(uint32_t max_elements, uint32_t num
 gms_status gms_multisplit_wide(const void* d_key_in, const void* d_value_in, void* d_key_out, void* d_value_out,
                                uint32_t n, int key_bytes, int value_bytes, const gms_bucket_desc64* desc,
                                void* d_scratch, size_t scratch_bytes, uint32_t* h_offsets, gms_stream_t stream) {
-  uint32_t* starts = h_offsets != nullptr && n != 0 ? t_starts.get() : nullptr;
+  uint32_t* starts = nullptr;
   gms_status st = multisplit_wide_impl(d_key_in, d_value_in, d_key_out, d_value_out, n, key_bytes, value_bytes, desc,
-                                       d_scratch, scratch_bytes, stream, starts,
-                                       h_offsets != nullptr && starts == nullptr);
+                                       d_scratch, scratch_bytes, stream, h_offsets != nullptr ? &starts : nullptr);
   if (st != GMS_SUCCESS || h_offsets == nullptr) return st;
   int logb = 0;
   valid_buckets(desc->num_buckets, &logb);

@@ -15,9 +15,13 @@
  *
  * Scratch: the reference's contexts cudaMalloc a bucket-count matrix plus CUB
  * scan storage (src/api/multisplit.cuh:50-74).  Here the caller owns one
- * scratch buffer whose size *_scratch_bytes() reports; the library never
- * allocates.  A scratch buffer serves one call at a time (calls that overlap
- * on the GPU and share a buffer race).
+ * scratch buffer whose size *_scratch_bytes() reports; the library allocates no
+ * device memory for a call.  A call that returns bucket starts or a count to the
+ * host uses 1 KB of pinned host memory, held by the calling thread until it ends:
+ * the library allocates it 64 KB at a time, at most 1 MB in a CUDA context, and
+ * keeps it for later threads; threads beyond that get a plain copy.  A scratch
+ * buffer serves one call at a time (calls that overlap on the GPU and share a
+ * buffer race).
  */
 #ifndef GPUMULTISPLIT_H_
 #define GPUMULTISPLIT_H_
