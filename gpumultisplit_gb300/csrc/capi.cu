@@ -766,12 +766,12 @@ cudaError_t run_scan(uint32_t* data, uint32_t m, uint64_t* status, ScratchHeader
 cudaError_t run_scan_rows(uint32_t* rows, uint32_t num_buckets, uint32_t num_tiles, uint32_t per, uint64_t* status,
                           ScratchHeader* hdr, cudaStream_t stream) {
   const uint32_t ranges = (num_tiles + per - 1) / per;
-  const uint32_t blocks = num_buckets > SCAN_ROWS_COLS ? num_buckets / SCAN_ROWS_COLS : 1u;
+  const uint32_t blocks = num_buckets / SCAN_ROWS_COLS;
   return launch_after_previous(scan_rows_kernel, dim3(blocks), dim3(SCAN_ROWS_THREADS), 0, stream, rows, num_buckets,
                                ranges, per, status, hdr);
 }
 
-uint32_t scan_rows_limit(uint32_t num_buckets) { return scan_rows_max_ranges(num_buckets); }
+uint32_t scan_rows_limit() { return SCAN_ROWS_MAX_RANGES; }
 
 void note_cuda_error(cudaError_t e) { g_last_cuda_error = int(e); }
 

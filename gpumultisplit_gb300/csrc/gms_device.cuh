@@ -393,8 +393,9 @@ __host__ __device__ constexpr bool kind_keeps_bucket_bytes(int kind, bool kv) {
   return kind == KIND_RANGE || (!kv && (kind == KIND_DIV || kind == KIND_EVEN_FLOAT));
 }
 
-// The fewest bucket bits at which counts may be kept as rows (counts_as_rows in ms_host.h).
+// The fewest bucket bits and tiles at which counts may be kept as rows (counts_as_rows in ms_host.h).
 constexpr int ROWS_MIN_LOGB = 7;
+constexpr uint32_t ROWS_MIN_TILES = 512;
 
 // Identifier policies: what the kernels need to know about a bucket
 // identifier.  DescPolicy covers the precompiled descriptor kinds; the drop-in

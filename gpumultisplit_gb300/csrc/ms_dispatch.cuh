@@ -51,9 +51,9 @@ inline uint32_t persistent_grid(Kernel k, int threads, uint32_t work, std::atomi
 }
 
 // A prescan's grid: no more blocks than ranges that one scan of the rows takes.
-inline uint32_t rows_grid(uint32_t grid, const uint32_t* rows, uint32_t num_buckets) {
+inline uint32_t rows_grid(uint32_t grid, const uint32_t* rows) {
   if (rows == nullptr) return grid;
-  const uint32_t most = scan_rows_limit(num_buckets);
+  const uint32_t most = scan_rows_limit();
   return grid < most ? grid : most;
 }
 
@@ -268,7 +268,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
     if (stages & STAGE_PRESCAN) {
       static std::atomic<int> per_sm{0};
       auto kern = prescan64_kernel<C, P>;
-      const uint32_t grid = rows_grid(persistent_grid(kern, C::THREADS, g.num_tiles, per_sm), rows, C::B);
+      const uint32_t grid = rows_grid(persistent_grid(kern, C::THREADS, g.num_tiles, per_sm), rows);
       choose_rows(grid);
       kern<<<grid, C::THREADS, 0, stream>>>(kin, n, g.num_tiles, counts, params, hdr, status, g.num_chunks,
                                             bucket_bytes, rows_per);
@@ -297,7 +297,7 @@ cudaError_t launch_multisplit(const ElemT<KW>* kin, const ElemT<VW>* vin, ElemT<
   if (stages & STAGE_PRESCAN) {
     static std::atomic<int> per_sm{0};
     auto kern = prescan_kernel<C, P>;
-    const uint32_t grid = rows_grid(persistent_grid(kern, C::THREADS, g.num_tiles, per_sm), rows, C::B);
+    const uint32_t grid = rows_grid(persistent_grid(kern, C::THREADS, g.num_tiles, per_sm), rows);
     choose_rows(grid);
     kern<<<grid, C::THREADS, 0, stream>>>(kin, n, g.num_tiles, counts, params, hdr, status, g.num_chunks,
                                           bucket_bytes, rows_per);
@@ -571,7 +571,7 @@ cudaError_t digit_prescan_scan_t(const DigitPass& c, uint32_t* rows_per, bool* d
   static std::atomic<int> per_sm{0};
   auto kern = prescan_kernel<C, DigitPolicy<KIND, LOGB>>;
   uint32_t* const rows = counts_as_rows(LOGB, g.num_tiles) ? matrix : nullptr;  // nothing reads the matrix afterwards
-  const uint32_t grid = rows_grid(persistent_grid(kern, C::THREADS, g.num_tiles, per_sm), rows, C::B);
+  const uint32_t grid = rows_grid(persistent_grid(kern, C::THREADS, g.num_tiles, per_sm), rows);
   *rows_per = rows != nullptr ? (g.num_tiles + grid - 1) / grid : 0u;
   kern<<<grid, C::THREADS, 0, c.stream>>>(c.kin, c.n, g.num_tiles, matrix, c.bp, hdr, status, g.num_chunks,
                                           c.bucket_bytes, *rows_per);

@@ -87,7 +87,9 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // rows: 2^25 keys 64 buckets 102 / 102, 128 116 / 109, 256 148 / 123; pairs 32
 // buckets 116 / 121, 64 125 / 127, 128 138 / 137, 256 183 / 165), and from 512
 // tiles up; fewer run as one launch where they can, and over the matrix where not.
-constexpr bool counts_as_rows(int logb, uint32_t num_tiles) { return logb >= ROWS_MIN_LOGB && num_tiles >= 512; }
+constexpr bool counts_as_rows(int logb, uint32_t num_tiles) {
+  return logb >= ROWS_MIN_LOGB && num_tiles >= ROWS_MIN_TILES;
+}
 
 // Scratch layout of one multisplit: [header 256 B][count matrix u32 x B*tiles][scan status u64 x chunks].
 // The matrix always starts at byte 256, whatever n is.
@@ -252,10 +254,10 @@ cudaError_t launch_after_previous(void (*kern)(KArgs...), dim3 grid, dim3 block,
 }
 
 // Scans the range totals in a prescan's rows (scan_kernels.cuh); at most
-// scan_rows_limit(num_buckets) ranges.
+// scan_rows_limit() ranges.
 cudaError_t run_scan_rows(uint32_t* rows, uint32_t num_buckets, uint32_t num_tiles, uint32_t per, uint64_t* status,
                           ScratchHeader* hdr, cudaStream_t stream);
-uint32_t scan_rows_limit(uint32_t num_buckets);
+uint32_t scan_rows_limit();
 
 cudaError_t run_scan(uint32_t* data, uint32_t m, uint64_t* status, ScratchHeader* hdr, cudaStream_t stream);
 

@@ -35,10 +35,11 @@ constexpr int SCAN_ROWS_THREADS = 1024;
 constexpr uint32_t SCAN_ROWS_COLS = 8;
 constexpr uint32_t SCAN_ROWS_KEEP = 10;  // ranges a thread holds in registers
 
-// The most ranges one launch scans.
-constexpr uint32_t scan_rows_max_ranges(uint32_t num_buckets) {
-  return SCAN_ROWS_KEEP * (uint32_t(SCAN_ROWS_THREADS) / (num_buckets < SCAN_ROWS_COLS ? num_buckets : SCAN_ROWS_COLS));
-}
+constexpr uint32_t SCAN_ROWS_GROUPS = SCAN_ROWS_THREADS / SCAN_ROWS_COLS;  // threads per column
+constexpr uint32_t SCAN_ROWS_MAX_RANGES = SCAN_ROWS_KEEP * SCAN_ROWS_GROUPS;
+static_assert((1u << ROWS_MIN_LOGB) % SCAN_ROWS_COLS == 0, "whole blocks of buckets");
+// The prescan resets a status word per SCAN_CHUNK counts; every block here uses one.
+static_assert(ROWS_MIN_TILES * SCAN_ROWS_COLS >= SCAN_CHUNK, "a reset status word for every block");
 
 __global__ void __launch_bounds__(SCAN_ROWS_THREADS) scan_rows_kernel(uint32_t* __restrict__ rows, uint32_t num_buckets,
                                                                       uint32_t ranges, uint32_t per,
@@ -54,8 +55,8 @@ __global__ void __launch_bounds__(SCAN_ROWS_THREADS) scan_rows_kernel(uint32_t* 
   __syncthreads();
   const uint32_t blk = s_blk;
   if (blk >= gridDim.x) return;
-  const uint32_t cols = min(num_buckets, SCAN_ROWS_COLS);
-  const uint32_t groups = SCAN_ROWS_THREADS / cols;  // threads per column, a multiple of 32
+  constexpr uint32_t cols = SCAN_ROWS_COLS, groups = SCAN_ROWS_GROUPS;
+  static_assert(groups % 32 == 0, "a warp scans whole slots of a column's threads");
   const uint32_t c = tid % cols, r = tid / cols;
   const uint32_t each = (ranges + groups - 1) / groups;
   const size_t stride = size_t(per) * num_buckets;
