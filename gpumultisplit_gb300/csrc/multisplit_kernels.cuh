@@ -275,7 +275,7 @@ __host__ __device__ inline uint32_t prescan_tiles_per_block(uint32_t num_tiles, 
 // 115, 128 135 / 118).  A splitter search is bound by its longest range (256
 // buckets, 2^28 keys 330 / 340).
 template <class P>
-constexpr bool prescan_whole_groups() {
+__host__ __device__ constexpr bool prescan_whole_groups() {
   return !P::USES_SMEM;
 }
 
