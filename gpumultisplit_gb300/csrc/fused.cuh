@@ -21,7 +21,26 @@ enum FusedSync : uint32_t {
   FUSED_ONE_TILE = 0,  // a single block: nothing to wait for
   FUSED_CLUSTER = 1,   // one thread-block cluster: the hardware's cluster barrier
   FUSED_GRID = 2,      // a cooperative launch: all blocks are resident, so the grid barrier ends
+  FUSED_NONE = 3,      // they cannot: not one launch
 };
+
+constexpr uint32_t FUSED_CLUSTER_MAX = 16;  // blocks of one cluster (above 8: opt-in)
+
+// How num_tiles tiles that are resident at once meet.  cluster_placed: the device
+// can place a cluster of their size; has_rows: there is room for their counts,
+// which only a cluster can do without.
+inline uint32_t fused_sync_of(uint32_t num_tiles, bool cluster_placed, bool has_rows) {
+  if (num_tiles == 1) return FUSED_ONE_TILE;
+  if (num_tiles <= FUSED_CLUSTER_MAX && cluster_placed) return FUSED_CLUSTER;
+  return has_rows ? FUSED_GRID : FUSED_NONE;
+}
+
+// Launch errors that say that this device (or the part of it that the process
+// may use) has no room for the launch's form; the stages run instead.
+inline bool fused_declined(cudaError_t e) {
+  return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorInvalidClusterSize ||
+         e == cudaErrorLaunchOutOfResources;
+}
 
 struct FusedArgs {
   uint32_t num_tiles;

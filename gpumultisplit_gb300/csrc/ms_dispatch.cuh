@@ -90,62 +90,77 @@ using ElemT = std::conditional_t<W == 2, uint64_t, uint32_t>;
 // against 10.5.
 constexpr uint32_t FUSED_CHEAP_PAIR_TILES = 448;
 constexpr uint32_t FUSED_ADD_MAX = 8192;
-constexpr uint32_t FUSED_CLUSTER_MAX = 16;  // blocks of one cluster (above 8: opt-in)
 
-// What a one-launch kernel remembers per process (per device where it matters).
+// What a one-launch kernel remembers per process; a bit per device, and per
+// cluster size (2, 4, 8, 16) whether a cluster of that size can be placed.
 struct FusedKernelState {
-  std::atomic<uint64_t> smem_done{0}, cluster_done{0};
+  std::atomic<uint64_t> smem_done{0};
+  std::atomic<uint64_t> placed[4] = {};
+  std::atomic<uint64_t> not_placed[4] = {};
   std::atomic<int> per_sm{0};
 };
 
+// Whether the current device can place the cluster that cfg describes.
+template <class Kernel>
+bool cluster_placed(Kernel kern, const cudaLaunchConfig_t& cfg, uint32_t blocks, FusedKernelState& state) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const uint64_t bit = 1ull << (dev & 63);
+  const int size = blocks <= 2 ? 0 : blocks <= 4 ? 1 : blocks <= 8 ? 2 : 3;
+  if (state.placed[size].load(std::memory_order_acquire) & bit) return true;
+  if (state.not_placed[size].load(std::memory_order_acquire) & bit) return false;
+  int clusters = 0;
+  const bool yes =
+      (blocks <= 8 || cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+      cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters > 0;
+  if (!yes) cudaGetLastError();
+  (yes ? state.placed : state.not_placed)[size].fetch_or(bit, std::memory_order_acq_rel);
+  return yes;
+}
+
 // Prepares `kern` to run num_tiles tiles in one launch: its limits, the form of
 // its barrier (a->sync) and the launch configuration.  *fits: all tiles are
-// resident at once.
+// resident at once and can meet.
 template <class C, class Kernel>
 cudaError_t fused_config(Kernel kern, size_t smem, size_t static_smem, uint32_t num_tiles, FusedKernelState& state,
                          cudaStream_t stream, FusedArgs* a, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr,
                          bool* fits) {
   *fits = false;
-  cudaError_t e = ensure_smem_limit(kern, smem, state.smem_done, static_smem);
+  const cudaError_t e = ensure_smem_limit(kern, smem, state.smem_done, static_smem);
   if (e != cudaSuccess) return e;
   if (persistent_grid(kern, C::THREADS, num_tiles, state.per_sm, smem) < num_tiles) return cudaSuccess;
   a->num_tiles = num_tiles;
-  a->sync = num_tiles == 1 ? FUSED_ONE_TILE : num_tiles <= FUSED_CLUSTER_MAX ? FUSED_CLUSTER : FUSED_GRID;
-  uint32_t blocks = num_tiles;
+  cfg->blockDim = dim3(C::THREADS);
+  cfg->dynamicSmemBytes = smem;
+  cfg->stream = stream;
   cfg->attrs = attr;
-  if (a->sync == FUSED_CLUSTER) {
-    for (blocks = 2; blocks < num_tiles; blocks <<= 1) {
-    }
+  bool placed = false;
+  if (num_tiles > 1 && num_tiles <= FUSED_CLUSTER_MAX) {
+    uint32_t blocks = 2;
+    while (blocks < num_tiles) blocks <<= 1;
     attr->id = cudaLaunchAttributeClusterDimension;
     attr->val.clusterDim.x = blocks;
     attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
     cfg->numAttrs = 1;
-    int dev = 0;
-    e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    const uint64_t bit = 1ull << (dev & 63);
-    if (blocks > 8 && !(state.cluster_done.load(std::memory_order_acquire) & bit)) {
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e != cudaSuccess) return e;
-      state.cluster_done.fetch_or(bit, std::memory_order_acq_rel);
-    }
-  } else if (a->sync == FUSED_GRID) {
+    cfg->gridDim = dim3(blocks);
+    placed = cluster_placed(kern, *cfg, blocks, state);
+  }
+  a->sync = fused_sync_of(num_tiles, placed, a->rows != nullptr);
+  if (a->sync == FUSED_NONE) return cudaSuccess;
+  if (a->sync != FUSED_CLUSTER) {
+    cfg->gridDim = dim3(num_tiles);
     attr->id = cudaLaunchAttributeCooperative;
     attr->val.cooperative = 1;
-    cfg->numAttrs = 1;
+    cfg->numAttrs = a->sync == FUSED_GRID ? 1 : 0;
   }
-  cfg->gridDim = dim3(blocks);
-  cfg->blockDim = dim3(C::THREADS);
-  cfg->dynamicSmemBytes = smem;
-  cfg->stream = stream;
   *fits = true;
   return cudaSuccess;
 }
 
-// The outcome of a one-launch kernel's launch: one refused because the device
-// offers fewer SMs than it has is not an error, the stages run instead.
+// The outcome of a one-launch kernel's launch: one that the device has no room
+// for is not an error, the stages run instead.
 inline cudaError_t fused_launched(cudaError_t e, bool* launched) {
-  *launched = e != cudaErrorCooperativeLaunchTooLarge;
+  *launched = !fused_declined(e);
   if (*launched) return e;
   cudaGetLastError();
   return cudaSuccess;
