@@ -114,9 +114,9 @@ cudaError_t run_batch_warp_kind(int kind, const BatchClassLaunch& c) {
 // of 16 to 1 Mi pairs with four, 283 with eight); one more for the one-warp classes.
 constexpr int kSideStreams = 4;
 
+// A creation that failed leaves what was made; the next run makes the rest.
 cudaError_t ensure_side_streams(gms_batch_s* b) {
-  if (!b->side.empty()) return cudaSuccess;
-  for (int i = 0; i < kSideStreams + 1; ++i) {
+  while (b->side.size() < size_t(kSideStreams) + 1) {
     cudaStream_t st = nullptr;
     cudaEvent_t ev = nullptr;
     cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
@@ -128,8 +128,9 @@ cudaError_t ensure_side_streams(gms_batch_s* b) {
     b->side.push_back(st);
     b->events.push_back(ev);
   }
+  if (b->events.size() > b->side.size()) return cudaSuccess;
   cudaEvent_t fork = nullptr;
-  cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+  const cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
   if (e == cudaSuccess) b->events.push_back(fork);  // last event: the fork point
   return e;
 }
