@@ -614,6 +614,66 @@ __device__ __forceinline__ void rows_to_matrix(const uint32_t* __restrict__ rows
   }
 }
 
+// Phase 4 of a tile ranked by atomics: calls store(p, source, bucket) for every
+// sorted position p < cnt of the staged tile.  Each warp stores runs of RUN times
+// 32 positions and checks beside it that (bucket, source) ascends from each
+// position to the next, by a shuffle; from run to run one thread each checks.  If
+// it does not somewhere in the tile, every bucket's run is put in order and the
+// tile is stored again.
+// Longer runs leave fewer places between them to check (the 7-bit sort of 2^25
+// keys: 551 us at one, 543 at four); at 256 buckets, whose runs are shortest,
+// pairs want the block's stores close together (the 8-bit sort of 2^25 pairs: 606
+// us at one, 638 at four).
+template <class C, class P, bool FULL, bool GIVEN, class Store>
+__device__ __forceinline__ void store_in_order(uint32_t cnt, const typename P::Id& ident, unsigned char* smem,
+                                               Store store) {
+  using L = PostLayout<C, P, GIVEN>;
+  using IndexT = std::conditional_t<L::WORDS, uint32_t, uint16_t>;
+  constexpr int IPT = C::IPT;
+  constexpr uint32_t B = C::B;
+  constexpr uint32_t RUN = C::KV && C::LOGB == 8 ? 1 : 4;
+  const typename C::KT* s_k = reinterpret_cast<const typename C::KT*>(smem + L::OFF_K);
+  IndexT* s_idx = reinterpret_cast<IndexT*>(smem + L::OFF_R);
+  const uint8_t* s_rb = reinterpret_cast<const uint8_t*>(smem + L::OFF_RB);
+  const typename L::WhT* s_wh = reinterpret_cast<const typename L::WhT*>(smem + L::OFF_WH);
+  const uint32_t tid = threadIdx.x;
+  const uint32_t lane = tid & 31u;
+  const uint32_t warp = tid >> 5;
+  // (bucket << 16) | source of sorted position p.
+  auto entry = [&](uint32_t p) -> uint32_t {
+    const uint32_t e = s_idx[p];
+    if constexpr (L::WORDS)
+      return e;
+    else if constexpr (L::BUCKET_BYTES)
+      return (uint32_t(s_rb[p]) << 16) | e;
+    else
+      return (ident(s_k[e]) << 16) | e;
+  };
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    bool late = false;
+    uint32_t before = 0;  // lane 0: entry of the position before its slot
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+      const uint32_t p = (uint32_t(j) / RUN * C::WARPS + warp) * (32u * RUN) + uint32_t(j) % RUN * 32u + lane;
+      uint32_t at = ~0u;
+      if (FULL || p < cnt) {
+        at = entry(p);
+        store(p, at & 0xFFFFu, at >> 16);
+      }
+      const uint32_t left = __shfl_sync(~0u, at, (lane + 31u) & 31u);
+      late |= (lane != 0 ? left : j % RUN == 0 ? 0u : before) > at;
+      before = left;
+    }
+    for (uint32_t p = 32u * RUN * (tid + 1u); p < cnt; p += 32u * RUN * C::THREADS) late |= entry(p - 1) > entry(p);
+    if (!__syncthreads_or(late)) break;
+    if (tid < B) {  // s_wh[b] of warp 0 is the start of bucket b's run
+      const uint32_t first = s_wh[tid], last = tid + 1 < B ? uint32_t(s_wh[tid + 1]) : cnt;
+      sort_run(s_idx + first, last - first);
+    }
+    __syncthreads();
+  }
+}
+
 // Phases 1-4 of the postscan for one staged tile.  FULL: the tile holds
 // exactly TILE keys, so no per-key validity test is needed.
 //
@@ -882,51 +942,8 @@ __device__ __forceinline__ bool postscan_tile(typename C::KT* __restrict__ kout,
     }
   };
   if constexpr (C::ATOMIC) {
-    // Each warp stores runs of RUN times 32 positions and checks beside it that
-    // (bucket, source) ascends from each position to the next, by a shuffle;
-    // from run to run one thread each checks.  If it does not somewhere in the
-    // tile, every bucket's run is put in order and the tile is stored again.
-    // Longer runs leave fewer places between them to check (the 7-bit sort of
-    // 2^25 keys: 551 us at one, 543 at four); at 256 buckets, whose runs are
-    // shortest, pairs want the block's stores close together (the 8-bit sort of
-    // 2^25 pairs: 606 us at one, 638 at four).
-    constexpr uint32_t RUN = C::KV && LOGB == 8 ? 1 : 4;
-    using IndexT = std::conditional_t<L::WORDS, uint32_t, uint16_t>;
-    IndexT* s_idx = reinterpret_cast<IndexT*>(s_r);
-    // (bucket << 16) | source of sorted position p.
-    auto entry = [&](uint32_t p) -> uint32_t {
-      const uint32_t e = s_idx[p];
-      if constexpr (L::WORDS)
-        return e;
-      else if constexpr (L::BUCKET_BYTES)
-        return (uint32_t(s_rb[p]) << 16) | e;
-      else
-        return (ident(s_k[e]) << 16) | e;
-    };
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      bool late = false;
-      uint32_t before = 0;  // lane 0: entry of the position before its slot
-#pragma unroll
-      for (int j = 0; j < IPT; ++j) {
-        const uint32_t p = (uint32_t(j) / RUN * C::WARPS + warp) * (32u * RUN) + uint32_t(j) % RUN * 32u + lane;
-        uint32_t at = ~0u;
-        if (FULL || p < cnt) {
-          at = entry(p);
-          const uint32_t src = at & 0xFFFFu;
-          store(p, src, s_k[src], at >> 16);
-        }
-        const uint32_t left = __shfl_sync(~0u, at, (lane + 31u) & 31u);
-        late |= (lane != 0 ? left : j % RUN == 0 ? 0u : before) > at;
-        before = left;
-      }
-      for (uint32_t p = 32u * RUN * (tid + 1u); p < cnt; p += 32u * RUN * C::THREADS) late |= entry(p - 1) > entry(p);
-      if (!__syncthreads_or(late)) break;
-      if (tid < B) {  // s_wh[b] of warp 0 is the start of bucket b's run
-        const uint32_t first = s_wh[tid], last = tid + 1 < B ? uint32_t(s_wh[tid + 1]) : cnt;
-        sort_run(s_idx + first, last - first);
-      }
-      __syncthreads();
-    }
+    store_in_order<C, P, FULL, GIVEN>(cnt, ident, smem,
+                                      [&](uint32_t p, uint32_t src, uint32_t b) { store(p, src, s_k[src], b); });
     return true;
   }
 #pragma unroll
