@@ -120,15 +120,17 @@ uint64_t current_context_id() {
   return id + 1;
 }
 
+ThreadStarts& this_thread_starts() {
+  static StartsPool& pool = *new StartsPool(alloc_pinned_words);  // outlives every thread
+  thread_local ThreadStarts mine(pool);
+  return mine;
+}
+
 // The calling thread's pinned words for a call that returns bucket starts, or
 // null (the caller then copies the matrix).  Against a strided device-to-host
 // copy of column 0 after the kernels, a call of 10 k pairs at 32 buckets took 19
 // us instead of 24, without the copy's own latency.
-uint32_t* thread_starts() {
-  static StartsPool& pool = *new StartsPool(alloc_pinned_words);  // outlives every thread
-  thread_local ThreadStarts mine(pool);
-  return mine.get(current_context_id());
-}
+uint32_t* thread_starts() { return this_thread_starts().get(current_context_id()); }
 
 // Shared body of the multisplit entry points (stage mask selects the kernels).
 // starts (or null): receives the words in which the last kernel leaves the
@@ -179,7 +181,10 @@ gms_status copy_offsets(const void* scratch, uint32_t n, int logb, uint32_t B, b
   }
   if (starts != nullptr) {
     const cudaError_t e = cudaStreamSynchronize(stream);
-    if (e == cudaSuccess) std::memcpy(h_offsets, starts, size_t(B) * sizeof(uint32_t));
+    if (e == cudaSuccess)
+      std::memcpy(h_offsets, starts, size_t(B) * sizeof(uint32_t));
+    else
+      this_thread_starts().abandon();
     return cuda_status(e);
   }
   const Geometry g = make_geometry(n, logb, kv, kw, vw);

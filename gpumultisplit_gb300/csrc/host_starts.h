@@ -1,6 +1,8 @@
 // Pinned host words in which a call's last kernel leaves the bucket starts for
 // the host (capi.cu).  A call that returns starts waits for its stream before
-// it returns, so a thread's words serve one call at a time.
+// it returns, so a thread's words serve one call at a time; where the wait fails
+// (another thread captures a stream in the global mode) its kernel may still run,
+// and the words are given up.
 //
 // Words belong to the CUDA context in which they were allocated and vanish with
 // it (cudaDeviceReset), so slots are kept per context.  Threads hand their slot
@@ -91,6 +93,9 @@ class ThreadStarts {
     context_ = context;
     return slot_;
   }
+
+  // Drops the slot for good: a kernel that nobody waited for may still write it.
+  void abandon() noexcept { slot_ = nullptr; }
 
  private:
   void release() noexcept {
