@@ -418,8 +418,8 @@ def set_sort_method(method: str) -> None:
     """How the 32-bit radix sorts run their digits, process-wide: "multisplit"
     (prescan, scan, postscan per digit, the reference's way), "onesweep" (one
     histogram pass, then one look-back pass per digit) or "auto" (the
-    library's choice, at present the multisplit passes).  The output is the
-    same either way."""
+    library's choice: one launch up to 2.49 M keys, the multisplit passes
+    above).  The output is the same whatever the method."""
     check(_lib.load().gms_sort_set_method(SORT_METHODS[method]), "gms_sort_set_method")
 
 

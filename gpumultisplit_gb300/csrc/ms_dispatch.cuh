@@ -84,6 +84,14 @@ using ElemT = std::conditional_t<W == 2, uint64_t, uint32_t>;
 // Larger inputs keep the memory busier as three stages, whose tiles are in
 // different phases.
 //
+// Beside large calls on another stream (2^28 pairs into 256 buckets) a small one
+// waits for room, three stages three times, one launch once (us until it is done,
+// three stages / one launch):
+//   keys, 256 buckets    3 k 675 -> 350   50 k 590 -> 320   130 k 895 -> 69   1 Mi 725 -> 49   2.4 M 950 -> 52
+//   pairs, 32 buckets   10 k 705 -> 455  300 k 755 -> 71     1 Mi 803 -> 49
+// A cooperative grid, from 17 tiles up, seems to be placed ahead of the blocks that
+// the large kernel has left.  The large calls take the same time.
+//
 // Up to FUSED_ADD_MAX counts every block adds up the rows itself (one
 // barrier); above, the columns are scanned first (two barriers).  At 256
 // buckets: 130 k keys (8192 counts) 10.1 against 11.6 us, 260 k keys 11.7

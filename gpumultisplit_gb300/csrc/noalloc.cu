@@ -15,10 +15,9 @@
 //     multisplit's minimum scratch (header, count matrix and scan status, without
 //     the optional byte per key) fits: up to 16,764,928 pairs at 256 buckets
 //     (4093 tiles of 4096), proportionally more at fewer buckets.  Larger calls
-//     are rejected with GMS_ERROR_SCRATCH_TOO_SMALL.  Costly identifiers (range,
-//     div, even-float) keep their byte per key in the array only when it also
-//     fits, and otherwise evaluate the identifier in both stages; the output is
-//     the same either way.  More than 256 buckets take two digit passes whose
+//     are rejected with GMS_ERROR_SCRATCH_TOO_SMALL.  Range identifiers
+//     keep their byte per key in the array only when it also fits, and otherwise
+//     are evaluated in both stages; the output is the same either way.  More than 256 buckets take two digit passes whose
 //     ping-pong keys and values also live in the array (about 460 thousand pairs
 //     at 1000 buckets).
 //   * The first call on a device looks up the array's device address

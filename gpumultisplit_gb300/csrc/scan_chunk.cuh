@@ -42,8 +42,9 @@ __device__ __forceinline__ void scan_chunk(uint32_t* __restrict__ data, uint32_t
   // Lane l of warp w holds, for k < SCAN_IPT / 4, the four counts at
   // first + 128 k: a warp reads and writes whole 512-byte runs.  With 16
   // consecutive counts per lane each 16-byte access touched a sector of its
-  // own: a 12.3 M-key call at 256 buckets took 68.2 us, now 67.1; 2^25 pairs of
-  // 64-bit elements 282.2, now 279.9.
+  // own: a 12.3 M-key call at 256 buckets took 68.2 us, with whole runs 67.1;
+  // 2^25 pairs of 64-bit elements 282.2 and 279.9 (measured while one-call
+  // multisplits of 65 and more buckets scanned their matrix; they scan rows now).
   constexpr int NV = SCAN_IPT / 4;
   const uint32_t first = chunk * SCAN_CHUNK + warp * (32u * SCAN_IPT) + lane * 4u;
 

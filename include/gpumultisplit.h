@@ -192,7 +192,7 @@ gms_status gms_sort_7bit_key_value(const uint32_t* d_key_in, uint32_t* d_key_out
  * src/api/multisplit_sort_pairs.cuh:67-260), same schedules:
  *   4: eight 4-bit passes;  5: six 5-bit passes then bits [30,32);
  *   6: 4-bit, 4-bit, then four 6-bit passes;  7: as above;  8: four 8-bit passes.
- * Under GMS_SORT_AUTO a sort of up to 2.5 M keys runs as one launch, in 8-bit
+ * Under GMS_SORT_AUTO a sort of up to 2.49 M keys runs as one launch, in 8-bit
  * digits whatever the width; the sorted order is the same.  The reported size
  * then includes its counts (at most 0.6 MB); without them the passes run.
  * digit_bits outside 4..8 is GMS_ERROR_INVALID_VALUE. */
@@ -210,9 +210,10 @@ gms_status gms_sort_key_value(const uint32_t* d_key_in, uint32_t* d_key_out, con
  *   GMS_SORT_ONESWEEP    one histogram pass for every digit, then one pass per
  *                        digit whose tiles find their offsets by decoupled
  *                        look-back (no count matrix, no scan);
- *   GMS_SORT_AUTO        the library's choice (at present the multisplit
- *                        passes, which measured faster on GB300).
- * Both give bit-identical output and fit the same scratch size. */
+ *   GMS_SORT_AUTO        the library's choice: one launch for a small sort (see
+ *                        above), the multisplit passes for the others, which
+ *                        measured faster than one-sweep on GB300.
+ * All give bit-identical output and fit the same scratch size. */
 enum { GMS_SORT_AUTO = 0, GMS_SORT_MULTISPLIT = 1, GMS_SORT_ONESWEEP = 2 };
 gms_status gms_sort_set_method(int method);
 gms_status gms_sort_get_method(int* method);
